@@ -156,6 +156,7 @@ struct Group {
   Ops* ops = nullptr;
   std::vector<Inst*> members;
   int epb = 1;
+  bool warp = false;            // the warp-per-element kernel runs it
   int variant = kVariantAuto;   // set by the autotuner
   bool dirty = true;
   // Device tables, two buffers: a rebuild writes the buffer that no launch
@@ -278,9 +279,10 @@ struct Ensemble {
     g->mixed = mixed;
     g->flags = mixed ? 0 : flags;
     g->ops = o;
-    g->epb = pipe_elems_per_tile(nq);
     // The fast pipelined kernels need the factored lift.
     const bool exact = !mixed && (flags & SDG_FLAG_EXACT);
+    g->epb = batch_elems_per_tile(nq, mixed, exact, !o->lift_z.empty());
+    g->warp = warp_kernel(nq, mixed, exact, !o->lift_z.empty());
     const bool can_pipe = pipe_supported(nq, mixed ? kStageMixed2 : kStageF64) &&
                           pipe_supported(nq, mixed ? kStageMixed1 : kStageF64) &&
                           pipe_supported(nq, mixed ? kStageMixed3 : kStageF64) &&
@@ -380,6 +382,14 @@ struct Ensemble {
     const int ni = static_cast<int>(g->members.size());
     g->h_insts.assign(3L * std::max(ni, 1), BatchInst{});
     g->h_tiles.clear();
+    // The warp-per-element kernel takes shorter tiles as well: a small group
+    // spreads over the SMs.
+    int epb = g->epb;
+    if (g->warp) {
+      long total = 0;
+      for (Inst* I : g->members) total += I->ne;
+      epb = static_cast<int>(std::max(1L, std::min<long>(epb, (total + num_sms - 1) / num_sms)));
+    }
     for (int m = 0; m < ni; ++m) {
       Inst* I = g->members[m];
       const void* in[3] = {I->q0, I->qa, I->qb};
@@ -397,8 +407,8 @@ struct Ensemble {
         b.fscale = I->fsc;
         b.dt = I->dt;
       }
-      for (int e0 = 0; e0 < I->ne; e0 += g->epb)
-        g->h_tiles.push_back(BatchTile{m, e0, std::min(g->epb, I->ne - e0), 0});
+      for (int e0 = 0; e0 < I->ne; e0 += epb)
+        g->h_tiles.push_back(BatchTile{m, e0, std::min(epb, I->ne - e0), 0});
     }
     g->ntiles = static_cast<int>(g->h_tiles.size());
     const int b = g->cur ^ 1;  // the buffer no launch in flight reads
@@ -524,6 +534,8 @@ struct Ensemble {
   // The kernel variants a group's launches support.
   std::vector<int> candidates(const Group* g) const {
     std::vector<int> cands;
+    // One kernel whatever the variant: launched as the pipelined one.
+    if (g->warp) return {kVariantPipe};
     const bool can_pipe = pipe_supported(g->nq, g->mixed ? kStageMixed2 : kStageF64) &&
                           pipe_supported(g->nq, g->mixed ? kStageMixed1 : kStageF64) &&
                           pipe_supported(g->nq, g->mixed ? kStageMixed3 : kStageF64);

@@ -31,10 +31,15 @@ int pipe_info(int nq, int kind, int* epb) {
   return table[nq](kind, epb);
 }
 
-int pipe_elems_per_tile(int nq) {
+bool warp_kernel(int nq, bool mixed, bool exact, bool factored) {
+  int epb = 1;
+  return !mixed && !exact && factored && (pipe_info(nq, kStageF64, &epb) & 4) != 0;
+}
+
+int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored) {
   int epb = 1;
   pipe_info(nq, kTendF64, &epb);
-  return epb;
+  return warp_kernel(nq, mixed, exact, factored) ? kWarpElems : epb;
 }
 
 bool pipe_supported(int nq, int kind) {

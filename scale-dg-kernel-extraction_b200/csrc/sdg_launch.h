@@ -92,9 +92,14 @@ struct LaunchSpec {
   int batch_ntiles;
 };
 
-// Elements per tile of the pipelined kernel for a given order (the tile
-// size a batch's tile table must use).
-int pipe_elems_per_tile(int nq);
+// Elements per tile of the batched kernels for a given order and form (the
+// tile size a batch's tile table must use); `factored`: Lift_mat factorises.
+int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored);
+
+// Whether the fast FP64 form of this order runs the warp-per-element kernel
+// (sdg_tend_warp.cuh), whatever variant is asked for.
+bool warp_kernel(int nq, bool mixed, bool exact, bool factored);
+constexpr int kWarpElems = 7;  // its elements per tile
 
 // Whether the pipelined kernel can run kind `kind` at this order (its
 // shared-memory plan fits).

@@ -302,6 +302,8 @@ struct TendArgs {
   // One-tile-per-block kernel: block b prefetches into L2 the inputs of
   // block b + prefetch_dist (about one resident wave ahead); 0 disables.
   int prefetch_dist;
+  // Warp-per-element kernel: elements per tile of a single instance (1..7).
+  int tile_elems;
   // Batched launches (pipelined kernel only): per-instance arrays and a
   // table of element tiles.  Null for a single instance, whose tiles are
   // the consecutive elements elem0 .. elem0+nelem-1 of the arrays above.

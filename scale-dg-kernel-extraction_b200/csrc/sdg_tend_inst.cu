@@ -9,6 +9,7 @@
 #include "sdg_tend.cuh"
 #include "sdg_tend_pipe.cuh"
 #include "sdg_tend_split.cuh"
+#include "sdg_tend_warp.cuh"
 
 #ifndef SDG_NQ
 #error "SDG_NQ must be defined"
@@ -53,6 +54,35 @@ int launch_pipe(size_t smem, int ntiles, const LaunchSpec& s, const Args& a, con
   return static_cast<int>(cudaGetLastError());
 }
 
+// Launches the warp-per-element kernel: one block per SM, or one per tile
+// where there are fewer.
+template <auto KERN, int H, typename Args, typename Dm>
+int launch_warp(int ntiles, const LaunchSpec& s, const Args& a, const Dm& d) {
+  constexpr auto kern = KERN;
+  static DeviceSetup setup;  // per kernel and device
+  const int dev = setup_device();
+  if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
+  if (setup.slot[dev].load(std::memory_order_relaxed) == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(WarpPlan<H>::BYTES));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    setup.slot[dev].store(1, std::memory_order_relaxed);
+  }
+  if (ntiles <= 0) return 0;
+  const int grid = std::min(ntiles, s.num_sms > 0 ? s.num_sms : 148);
+  kern<<<grid, WarpPlan<H>::THREADS, WarpPlan<H>::BYTES, s.stream>>>(a, d);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// Warps per element of the warp-per-element kernel for a mesh of `per_sm`
+// elements per SM: the split forms while one round of tiles holds them (one
+// element a tile with four warps, three with two).  Measured, us per RK step
+// from the step graph with H = 1 / 2 / 4: 64 elements 18.8 / 16.6 / 12.5, 148
+// 20.7 / 16.6 / 14.5, 296 20.7 / 16.6 / 18.6, 444 20.7 / 18.6 / 22.7, 592 20.7
+// / 24.8 / 26.8, 1036 20.7 / 30.9 / 37.1.
+inline int warps_per_elem(int per_sm) { return per_sm <= 1 ? 4 : (per_sm <= 3 ? 2 : 1); }
+
 template <typename TQ, typename TV, typename TO, typename TC, bool EXACT,
           int ORDER, bool STAGE>
 int run(const LaunchSpec& s) {
@@ -78,6 +108,7 @@ int run(const LaunchSpec& s) {
   a.wait_spins = s.wait_spins ? s.wait_spins : kWaitSpins;
   a.inject_skip = s.inject_skip;
   a.prefetch_dist = 0;
+  a.tile_elems = 0;
   a.insts = static_cast<const BatchInst*>(s.batch_insts);
   a.tiles = static_cast<const BatchTile*>(s.batch_tiles);
   a.ntiles = s.batch_ntiles;
@@ -93,10 +124,39 @@ int run(const LaunchSpec& s) {
   // fast pipelined kernels need the factored lift; with a verbatim table a
   // fast launch takes the one-tile-per-block kernel.
   const size_t pipe_bytes = batch ? PB::BYTES : P::BYTES;
-  const bool can_pipe = pipe_bytes <= kPipeMaxSmem && pipe_bytes <= device_smem_optin() &&
+  constexpr bool WARP = kWarpKernel<NQ, TC, EXACT>;
+  const bool can_pipe = !WARP && pipe_bytes <= kPipeMaxSmem && pipe_bytes <= device_smem_optin() &&
                         (EXACT || s.lift_z != nullptr) &&
                         (batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) &&
                                    aligned(s.w) && aligned(s.escale) && aligned(s.fscale)));
+  // Fast FP64 at Nq = 8 with a factored lift: one warp per element, for
+  // every requested variant (bulk copies where the arrays are aligned).
+  if constexpr (WARP) {
+    if (s.lift_z != nullptr && WarpPlan<1>::BYTES <= device_smem_optin()) {
+      const bool vec = batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) && aligned(s.w) &&
+                                 aligned(s.out) && (s.q0 == nullptr || aligned(s.q0)));
+      const int sms = s.num_sms > 0 ? s.num_sms : 148;
+      const int per_sm = (s.nelem + sms - 1) / sms;
+      // Tiles of the most elements the warps take, or fewer where that leaves
+      // an SM without one.
+      auto tiles = [&](int most) {
+        a.tile_elems = std::max(1, std::min(most, per_sm));
+        return batch ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
+      };
+      if (!vec && !batch)
+        return launch_warp<tend_warp_kernel<STAGE, false, false, 1>, 1>(tiles(7), s, a, d);
+      if (batch) return launch_warp<tend_warp_kernel<STAGE, true, true, 1>, 1>(tiles(7), s, a, d);
+      // (A call without elements primes every form.)
+      const int h = warps_per_elem(per_sm);
+      int rc = 0;
+      if (h == 4 || s.nelem <= 0)
+        rc = launch_warp<tend_warp_kernel<STAGE, false, true, 4>, 4>(tiles(1), s, a, d);
+      if (rc == 0 && (h == 2 || s.nelem <= 0))
+        rc = launch_warp<tend_warp_kernel<STAGE, false, true, 2>, 2>(tiles(3), s, a, d);
+      if (rc != 0 || (h != 1 && s.nelem > 0)) return rc;
+      return launch_warp<tend_warp_kernel<STAGE, false, true, 1>, 1>(tiles(7), s, a, d);
+    }
+  }
   // The split-column kernel: orders with one element per tile.
   if constexpr (NQ >= 9) {
     constexpr int H = kSplitH<NQ>;
@@ -140,7 +200,7 @@ int run(const LaunchSpec& s) {
   const bool pipe =
       batch || ((s.variant == kVariantPipe || s.variant == kVariantAuto ||
                  s.variant == kVariantSplit || s.variant == kVariantTensor) && can_pipe);
-  if (pipe) {
+  if constexpr (!WARP) if (pipe) {
     const int ntiles =
         batch ? s.batch_ntiles : (s.nelem + PipeGeo<NQ>::EPB - 1) / PipeGeo<NQ>::EPB;
     if (batch)
@@ -207,7 +267,8 @@ int run(const LaunchSpec& s) {
 
 // Which persistent plans fit both the build's limit and the current
 // device's per-block opt-in: bit 0 the pipelined kernel, bit 1 the
-// split-column kernel (orders with one element per tile).
+// split-column kernel (orders with one element per tile), bit 2 the
+// warp-per-element kernel of the fast FP64 form.
 template <typename TQ, typename TV, typename TC, bool STAGE>
 int pipe_fits() {
   const size_t optin = device_smem_optin();
@@ -217,6 +278,9 @@ int pipe_fits() {
   if constexpr (NQ >= 9) {
     constexpr size_t sb = SplitPlan<NQ, kSplitH<NQ>, TQ, TV, TC, STAGE>::BYTES;
     if (sb <= kPipeMaxSmem && sb <= optin) r |= 2;
+  }
+  if constexpr (kWarpKernel<NQ, TC, false>) {
+    if (WarpPlan<1>::BYTES <= optin) r |= 4;
   }
   return r;
 }

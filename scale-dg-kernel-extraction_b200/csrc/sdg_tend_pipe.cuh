@@ -77,6 +77,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                : "memory");
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -271,22 +275,6 @@ struct LineIdx<8, 4> {
   static __device__ __forceinline__ int xl(int base, int l) { return base ^ l; }
   static __device__ __forceinline__ int yl_base(int a, int b) { return 72 * b + (a ^ (b & 3)); }
   static __device__ __forceinline__ int yl(int base, int l) { return base ^ (8 * l + 4 * (l >> 2)); }
-};
-
-// Line buffers of the tensor-core contractions (fast FP64, Nq = 8): eight
-// k-planes of 64, each an 8x8 (i,j) block in which
-//   x:  F_x(i,j) at px(i,j) = (j ^ h(i)) + 8i,  DxF(i,j) at qx(i,j) = (j ^ (i&6)) + 8i
-//   y:  F_y(i,j) at py(i,j) = (i ^ h(j)) + 8j,  DyF(i,j) at qy(i,j) = (i ^ (j&6)) + 8j
-// with h(n) = ((n&2) << 1) | ((n&4) >> 1).  The four patterns on each buffer
-// (column writes of F, B-fragment loads, 16-byte C-fragment stores, column
-// reads of the result) each put a half-warp's eight-byte accesses on 16
-// distinct bank pairs.
-struct TensorIdx8 {
-  static __device__ __forceinline__ int h(int n) { return ((n & 2) << 1) | ((n & 4) >> 1); }
-  static __device__ __forceinline__ int px(int i, int j) { return (j ^ h(i)) + 8 * i; }
-  static __device__ __forceinline__ int qx(int i, int j) { return (j ^ (i & 6)) + 8 * i; }
-  static __device__ __forceinline__ int py(int i, int j) { return (i ^ h(j)) + 8 * j; }
-  static __device__ __forceinline__ int qy(int i, int j) { return (i ^ (j & 6)) + 8 * j; }
 };
 
 // A (q_minus, un_minus) pair of a face node, stored in one 8- or 16-byte word.
@@ -538,10 +526,8 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
   constexpr int NP = G::NP;
   constexpr int EPB = G::EPB;
   constexpr int NS = P::NSTAGE;
-  // x/y line contractions on the tensor cores (fast FP64, Nq = 8).
-  constexpr bool TENSOR = kTensorLines<NQ, TC, EXACT>;
-  double da0 = 0.0, da1 = 0.0;  // this lane's A fragments of D
-  if constexpr (TENSOR) dmma_dfrag(D, &da0, &da1);
+  static_assert(!(NQ == 8 && sizeof(TC) == 8 && !EXACT),
+                "fast FP64 at Nq = 8: tend_warp_kernel");
 
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* slots = smem_raw;
@@ -846,14 +832,6 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
     if (active) {
       if constexpr (TCG) {
         // The lines come from the tensor cores; no column writes.
-      } else if constexpr (TENSOR) {
-        TC* px = sX + TensorIdx8::px(a, b);
-        TC* py = sY + TensorIdx8::py(a, b);
-#pragma unroll
-        for (int k = 0; k < NQ; ++k) {
-          px[NQ2 * k] = fx[k];
-          py[NQ2 * k] = fy[k];
-        }
       } else {
 #pragma unroll
         for (int k = 0; k < NQ; ++k) {
@@ -917,24 +895,6 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
         for (int i = 0; i < NQ; ++i) {
           sX[LI::xl(lbx, i)] = rx[i];
           sY[LI::yl(lby, i)] = ry[i];
-        }
-      } else if constexpr (TENSOR) {
-        // DMMA tiles: the element's two warps take four k-planes each; a
-        // plane is read and rewritten only by its warp.
-        const int lane = threadIdx.x & 31, g = lane >> 2, qd = lane & 3;
-        const int we = t >> 5;  // warp of the element
-        using TI = TensorIdx8;
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          TC* px = sX + NQ2 * (4 * we + kk);
-          TC* py = sY + NQ2 * (4 * we + kk);
-          double d0, d1;
-          // x: B(l, j) = F_x(l, j), C(i, j) = DxF(i, j) on this plane.
-          dmma_tile8(da0, da1, px[TI::px(qd, g)], px[TI::px(4 + qd, g)], &d0, &d1);
-          *reinterpret_cast<double2*>(px + TI::qx(g, 2 * qd)) = make_double2(d0, d1);
-          // y: B(l, i) = F_y(i, l), C(j, i) = DyF(i, j).
-          dmma_tile8(da0, da1, py[TI::py(g, qd)], py[TI::py(g, 4 + qd)], &d0, &d1);
-          *reinterpret_cast<double2*>(py + TI::qy(2 * qd, g)) = make_double2(d0, d1);
         }
       } else {
         const int lbx = LI::xl_base(a, b), lby = LI::yl_base(a, b);
@@ -1018,14 +978,8 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
       // ---- Phase 4: z-derivative, lift, combine, store ---------------------
       const TC e1 = ses[0], e2 = ses[1], e3 = ses[2];
       // This column's entry of the x/y results at node k.
-      auto xres = [&](int k) -> TC {
-        if constexpr (TENSOR) return sX[TensorIdx8::qx(a, b) + NQ2 * k];
-        else return sX[LI::colx(a, b, k)];
-      };
-      auto yres = [&](int k) -> TC {
-        if constexpr (TENSOR) return sY[TensorIdx8::qy(a, b) + NQ2 * k];
-        else return sY[LI::coly(a, b, k)];
-      };
+      auto xres = [&](int k) -> TC { return sX[LI::colx(a, b, k)]; };
+      auto yres = [&](int k) -> TC { return sY[LI::coly(a, b, k)]; };
       TC lxy[4];
       if constexpr (!EXACT) {
         lxy[0] = sL[b];
