@@ -164,6 +164,7 @@ struct Group {
   // serving loop) and makes it current.
   BatchInst* d_insts_buf[2] = {nullptr, nullptr};  // [3][inst_cap]
   BatchTile* d_tiles_buf[2] = {nullptr, nullptr};
+  unsigned char* d_maps_buf[2] = {nullptr, nullptr};  // [3][inst_cap] FieldMaps
   int inst_cap_buf[2] = {0, 0}, tile_cap_buf[2] = {0, 0};
   int cur = 0;
   BatchInst* d_insts = nullptr;  // the current buffer
@@ -195,6 +196,7 @@ struct Ensemble {
       for (int b = 0; b < 2; ++b) {
         if (g.second->d_insts_buf[b]) cudaFree(g.second->d_insts_buf[b]);
         if (g.second->d_tiles_buf[b]) cudaFree(g.second->d_tiles_buf[b]);
+        if (g.second->d_maps_buf[b]) cudaFree(g.second->d_maps_buf[b]);
       }
       if (g.second->stream) cudaStreamDestroy(g.second->stream);
       if (g.second->done) cudaEventDestroy(g.second->done);
@@ -416,6 +418,11 @@ struct Ensemble {
       if (g->d_insts_buf[b]) cudaFree(g->d_insts_buf[b]);
       g->inst_cap_buf[b] = std::max(ni, 2 * g->inst_cap_buf[b]);
       ENS_CUDA(cudaMalloc(&g->d_insts_buf[b], 3L * g->inst_cap_buf[b] * sizeof(BatchInst)));
+      if (g->warp && g->mixed) {
+        if (g->d_maps_buf[b]) cudaFree(g->d_maps_buf[b]);
+        g->d_maps_buf[b] = nullptr;
+        ENS_CUDA(cudaMalloc(&g->d_maps_buf[b], 3L * g->inst_cap_buf[b] * kFieldMapsBytes));
+      }
     }
     if (g->ntiles > g->tile_cap_buf[b]) {
       if (g->d_tiles_buf[b]) cudaFree(g->d_tiles_buf[b]);
@@ -433,6 +440,25 @@ struct Ensemble {
       std::vector<BatchInst> padded(3L * g->inst_cap);
       for (int st = 0; st < 3; ++st)
         for (int m = 0; m < ni; ++m) padded[st * g->inst_cap + m] = g->h_insts[st * ni + m];
+      if (g->d_maps_buf[b]) {
+        std::vector<unsigned char> maps(padded.size() * kFieldMapsBytes);
+        for (int st = 0; st < 3; ++st)
+          for (int m = 0; m < ni; ++m) {
+            const size_t x = static_cast<size_t>(st) * g->inst_cap + m;
+            BatchInst& bi = padded[x];
+            const void* in[4] = {bi.q, bi.u, bi.v, bi.w};
+            for (int f = 0; f < 4; ++f) {
+              alignas(64) unsigned char one[128];
+              int rc = encode_field_map(one, in[f], f == 0 && st == 0 ? 8 : 4,
+                                        g->members[m]->ne);
+              if (rc) return rc;
+              std::memcpy(&maps[x * kFieldMapsBytes + 128 * f], one, sizeof(one));
+            }
+            bi.maps = g->d_maps_buf[b] + x * kFieldMapsBytes;
+          }
+        ENS_CUDA(cudaMemcpy(g->d_maps_buf[b], maps.data(), maps.size(),
+                            cudaMemcpyHostToDevice));
+      }
       ENS_CUDA(cudaMemcpy(g->d_insts, padded.data(), padded.size() * sizeof(BatchInst),
                           cudaMemcpyHostToDevice));
       ENS_CUDA(cudaMemcpy(g->d_tiles, g->h_tiles.data(), g->h_tiles.size() * sizeof(BatchTile),

@@ -4,6 +4,7 @@
 // The fused tendency kernel itself lives in sdg_tend.cuh and is instantiated
 // per polynomial order by sdg_tend_inst.cu.
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -33,13 +34,45 @@ int pipe_info(int nq, int kind, int* epb) {
 
 bool warp_kernel(int nq, bool mixed, bool exact, bool factored) {
   int epb = 1;
-  return !mixed && !exact && factored && (pipe_info(nq, kStageF64, &epb) & 4) != 0;
+  return !exact && factored && (pipe_info(nq, mixed ? kStageMixed1 : kStageF64, &epb) & 4) != 0;
+}
+
+int encode_field_map(void* map, const void* base, int elem_bytes, long nelem) {
+  // cuTensorMapEncodeTiled through the runtime, so that the library does not
+  // link the driver.
+  using Fn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                          const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                          const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Fn encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &st) !=
+            cudaSuccess || st != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<Fn>(fn);
+  }();
+  if (!encode) return fail(SDG_ERR_CUDA, "the driver has no cuTensorMapEncodeTiled");
+  const cuuint32_t rows = 512 * elem_bytes / 128;  // per element
+  const cuuint64_t dim[2] = {128u / elem_bytes, static_cast<cuuint64_t>(rows) * nelem};
+  const cuuint64_t stride[1] = {128};
+  const cuuint32_t box[2] = {128u / elem_bytes, rows};
+  const cuuint32_t one[2] = {1, 1};
+  const CUresult r =
+      encode(static_cast<CUtensorMap*>(map),
+             elem_bytes == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+             2, const_cast<void*>(base), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return fail(SDG_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", static_cast<int>(r));
+  return SDG_OK;
 }
 
 int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored) {
   int epb = 1;
   pipe_info(nq, kTendF64, &epb);
-  return warp_kernel(nq, mixed, exact, factored) ? kWarpElems : epb;
+  return warp_kernel(nq, mixed, exact, factored) ? (mixed ? kWarpElems32 : kWarpElems) : epb;
 }
 
 bool pipe_supported(int nq, int kind) {
@@ -227,6 +260,9 @@ struct sdg_handle {
   void* vel[3] = {nullptr, nullptr, nullptr};
   double* vel64[3] = {nullptr, nullptr, nullptr};  // FP64 upload staging
   bool have_vel[3] = {false, false, false};
+  // Tensor maps of each stage's inputs, where the mixed form takes them.
+  bool has_maps = false;
+  alignas(64) unsigned char maps[3][kFieldMapsBytes];
   bool have_q = false;
 
   // Reductions.
@@ -463,6 +499,15 @@ int ensure_state(sdg_handle* h) {
     for (int d = 0; d < 3; ++d)
       if (!(h->vel64[d] = dev_alloc<double>(NA, &rc))) return rc;
   SDG_CUDA(cudaMemsetAsync(h->q0, 0, NA * sizeof(double), h->stream));
+  if (mixed(h) && warp_kernel(h->Nq, true, false, !h->lift_z.empty())) {
+    const void* q[3] = {h->q0, h->qa, h->qb};
+    for (int st = 0; st < 3; ++st)
+      for (int f = 0; f < 4; ++f)
+        if ((rc = encode_field_map(h->maps[st] + 128 * f, f == 0 ? q[st] : h->vel[f - 1],
+                                   f == 0 && st == 0 ? 8 : 4, h->Ne)))
+          return rc;
+    h->has_maps = true;
+  }
   return SDG_OK;
 }
 
@@ -495,6 +540,7 @@ int enqueue_stage_range(sdg_handle* h, int st, double dt, int e0, int n) {
   s.rk_a = ra[st];
   s.rk_b = rb[st];
   s.dt = dt;
+  s.field_maps = h->has_maps ? h->maps[st] : nullptr;
   s.elem0 = e0;
   s.nelem = n;
   return launch_tend(s);
@@ -519,6 +565,7 @@ int prime_stages(sdg_handle* h) {
     s.out = h->qa;
     s.pbase = h->direct_ok ? h->pb_direct : h->pb_halo;
     s.rk_a = st == 0 ? 0.0 : 0.5;
+    s.field_maps = h->has_maps ? h->maps[st] : nullptr;
     s.nelem = 0;
     int rc = launch_tend(s);
     if (rc) return rc;

@@ -79,11 +79,11 @@ bool lift_factor(const double* Lift, int Nq, std::vector<double>* expanded,
       spread = std::fmax(spread, std::fabs(Lift[Np * f + n] - ref));
     }
   if (!(spread <= kLiftFactorTol * mx)) return false;
-  lift_z->resize(2L * Nq);
-  for (int k = 0; k < Nq; ++k) {
-    (*lift_z)[k] = ex[Np * 4 + Nq2 * k];
-    (*lift_z)[Nq + k] = ex[Np * 5 + Nq2 * k];
-  }
+  lift_z->resize(6L * Nq);
+  const int faces[6] = {4, 5, 3, 1, 0, 2};  // -z, +z, -x, +x, -y, +y
+  for (int x = 0; x < 6; ++x)
+    for (int k = 0; k < Nq; ++k)
+      (*lift_z)[x * Nq + k] = ex[Np * faces[x] + stride[kFaceAxis[faces[x]]] * k];
   expanded->swap(ex);
   return true;
 }

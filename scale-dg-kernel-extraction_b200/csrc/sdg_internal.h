@@ -30,8 +30,8 @@ constexpr double kLiftFactorTol = 1e-13;
 // tensor-product nodes, Lift(i,j,k,f) depends only on the node index
 // along face f's normal; `expanded` receives the table rebuilt from the
 // first tangential row of each face (entry (i,j,k,f) = Lift at normal
-// index n, tangential indices 0) and `lift_z` the z-face factors as
-// lift_z[k] (face -z) and lift_z[Nq + k] (face +z).  Returns false (and
+// index n, tangential indices 0) and `lift_z` the factors l_f(n) of the faces
+// -z, +z, -x, +x, -y, +y, Nq each.  Returns false (and
 // leaves the outputs empty) when some entry differs from its factor by
 // more than kLiftFactorTol * max|Lift_mat|.
 bool lift_factor(const double* Lift, int Nq, std::vector<double>* expanded,

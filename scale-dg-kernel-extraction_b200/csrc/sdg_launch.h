@@ -75,10 +75,13 @@ struct LaunchSpec {
   int nelem;
   double rk_a, rk_b, dt;
   const double* D;     // row-major D(i,l), NQ*NQ
-  // Factored lift of the fast kernels: the z-face factors lz(k, f) for
-  // f = -z, +z ((2, NQ), host memory), given when `lift` holds the
+  // Factored lift of the fast kernels: the factors l_f(n) for f = -z, +z, -x,
+  // +x, -y, +y ((6, NQ), host memory), given when `lift` holds the
   // tensor-product factorisation of Lift_mat; null for the verbatim table.
   const double* lift_z;
+  // Tensor maps of q, u, v, w (kFieldMapsBytes, host memory) of the mixed form
+  // at the orders that take them (field_map_elems); null otherwise.
+  const void* field_maps;
   cudaStream_t stream;
   int variant;         // KernelVariant
   int* status;         // device status word (bounded-wait timeouts)
@@ -96,10 +99,20 @@ struct LaunchSpec {
 // tile size a batch's tile table must use); `factored`: Lift_mat factorises.
 int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored);
 
-// Whether the fast FP64 form of this order runs the warp-per-element kernel
-// (sdg_tend_warp.cuh), whatever variant is asked for.
+// Whether the fast FP64 or mixed form of this order runs a warp-per-element
+// kernel (sdg_tend_warp.cuh, sdg_tend_warp32.cuh), whatever variant is asked
+// for.
 bool warp_kernel(int nq, bool mixed, bool exact, bool factored);
-constexpr int kWarpElems = 7;  // its elements per tile
+// Elements per tile: FP64, mixed.
+constexpr int kWarpElems = 7;
+constexpr int kWarpElems32 = 11;
+
+// The four tensor maps of a stage's inputs, and one of them: the field of
+// nelem elements of 512 values (elem_bytes each) at `base` as rows of 128
+// bytes, box one element, 128-byte swizzle.  SDG_OK or an SDG_ERR_* status
+// with the thread's last error set.
+constexpr size_t kFieldMapsBytes = 512;
+int encode_field_map(void* map, const void* base, int elem_bytes, long nelem);
 
 // Whether the pipelined kernel can run kind `kind` at this order (its
 // shared-memory plan fits).

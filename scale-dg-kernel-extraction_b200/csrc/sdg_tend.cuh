@@ -125,7 +125,10 @@ struct SmemLayout {
 template <int NQ, typename TC>
 struct DMat {
   TC d[NQ * NQ];
-  TC lz[2 * NQ];  // z-face lift factors (-z, +z) of the factored fast lift
+  // Lift factors of the factored fast lift, faces (-z, +z), (-x, +x), (-y, +y).
+  TC lz[2 * NQ];
+  TC lx[2 * NQ];
+  TC ly[2 * NQ];
 };
 
 // Sum_{l} A(l)*B(l) in the reference's order (see header comment).
@@ -154,11 +157,11 @@ __device__ __forceinline__ T contract(FA A, FB B) {
 // Orders (NQ = p + 1) whose fast FP32 kernels advance the x and y lines of a
 // thread together with packed FMAs (contract2).  Measured per order on the
 // pipelined kernel (G DOF-updates/s, paired vs scalar): p = 3 104.2 / 102.5,
-// p = 7 146.7 / 140.7, p = 10 128.5 / 121.2, p = 11 111.4 / 102.3, p = 12
+// p = 10 128.5 / 121.2, p = 11 111.4 / 102.3, p = 12
 // 119.9 / 99.4; slower at p = 4, 5, 8 (101.5 / 106.0, 106.7 / 114.1,
 // 109.1 / 118.7), where the wider live range costs a resident block.
 template <int NQ>
-constexpr bool kPairedLinesPipe = NQ == 4 || NQ == 8 || NQ >= 11;
+constexpr bool kPairedLinesPipe = NQ == 4 || NQ >= 11;
 // The one-tile-per-block kernel, which the fast FP32 forms run at p >= 13:
 // p = 13 78.2 / 63.5, p = 14 81.9 / 78.1, p = 15 92.7 / 86.9.
 template <int NQ>
@@ -326,6 +329,7 @@ struct BatchInst {
   const void* escale;
   const void* fscale;
   double dt;
+  const void* maps;     // FieldMaps of (q, u, v, w), where the kernel takes them
 };
 
 // A tile: up to EPB consecutive elements e0 .. e0+n-1 of instance `inst`.

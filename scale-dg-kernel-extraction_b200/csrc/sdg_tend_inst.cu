@@ -4,12 +4,14 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstring>
 
 #include "sdg_launch.h"
 #include "sdg_tend.cuh"
 #include "sdg_tend_pipe.cuh"
 #include "sdg_tend_split.cuh"
 #include "sdg_tend_warp.cuh"
+#include "sdg_tend_warp32.cuh"
 
 #ifndef SDG_NQ
 #error "SDG_NQ must be defined"
@@ -75,6 +77,31 @@ int launch_warp(int ntiles, const LaunchSpec& s, const Args& a, const Dm& d) {
   return static_cast<int>(cudaGetLastError());
 }
 
+// The mixed form's warp-per-element kernel: tiles of the most elements a slot
+// holds, or fewer where that leaves an SM without one.
+template <auto KERN, typename TQ, int H, typename Args, typename Dm>
+int launch_warp32(const LaunchSpec& s, Args& a, const Dm& d, const FieldMaps& m) {
+  constexpr auto kern = KERN;
+  using P = Warp32Plan<TQ, H>;
+  static DeviceSetup setup;  // per kernel and device
+  const int dev = setup_device();
+  if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
+  if (setup.slot[dev].load(std::memory_order_relaxed) == 0) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(P::BYTES));
+    if (e != cudaSuccess) return static_cast<int>(e);
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    setup.slot[dev].store(1, std::memory_order_relaxed);
+  }
+  const int sms = s.num_sms > 0 ? s.num_sms : 148;
+  a.tile_elems = std::max(1, std::min(P::ELEMS, (s.nelem + sms - 1) / sms));
+  const int ntiles = s.batch_tiles ? s.batch_ntiles
+                                   : (s.nelem + a.tile_elems - 1) / a.tile_elems;
+  if (ntiles <= 0) return 0;
+  kern<<<std::min(ntiles, sms), P::THREADS, P::BYTES, s.stream>>>(a, d, m);
+  return static_cast<int>(cudaGetLastError());
+}
+
 // Warps per element of the warp-per-element kernel for a mesh of `per_sm`
 // elements per SM: the split forms while one round of tiles holds them (one
 // element a tile with four warps, three with two).  Measured, us per RK step
@@ -114,8 +141,11 @@ int run(const LaunchSpec& s) {
   a.ntiles = s.batch_ntiles;
   DMat<NQ, TC> d;
   for (int i = 0; i < NQ * NQ; ++i) d.d[i] = static_cast<TC>(s.D[i]);
-  for (int i = 0; i < 2 * NQ; ++i)
+  for (int i = 0; i < 2 * NQ; ++i) {
     d.lz[i] = s.lift_z ? static_cast<TC>(s.lift_z[i]) : TC(0);
+    d.lx[i] = s.lift_z ? static_cast<TC>(s.lift_z[2 * NQ + i]) : TC(0);
+    d.ly[i] = s.lift_z ? static_cast<TC>(s.lift_z[4 * NQ + i]) : TC(0);
+  }
   using P = PipePlan<NQ, TQ, TV, TC, STAGE>;
   using PB = PipePlan<NQ, TQ, TV, TC, STAGE, false, true>;  // batched launches
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -155,6 +185,27 @@ int run(const LaunchSpec& s) {
         rc = launch_warp<tend_warp_kernel<STAGE, false, true, 2>, 2>(tiles(3), s, a, d);
       if (rc != 0 || (h != 1 && s.nelem > 0)) return rc;
       return launch_warp<tend_warp_kernel<STAGE, false, true, 1>, 1>(tiles(7), s, a, d);
+    }
+  }
+  // The mixed form at Nq = 8, likewise (but for the tensor-core experiment).
+  if constexpr (STAGE && kWarp32Kernel<NQ, TC, EXACT>) {
+    if (s.lift_z != nullptr && (batch || s.field_maps != nullptr) &&
+        s.variant != kVariantTensor && Warp32Plan<TQ, 1>::BYTES <= device_smem_optin()) {
+      FieldMaps m;
+      std::memset(&m, 0, sizeof(m));
+      if (batch) return launch_warp32<tend_warp32_kernel<TQ, TO, true, 1>, TQ, 1>(s, a, d, m);
+      std::memcpy(&m, s.field_maps, sizeof(m));
+      // Two warps an element while one round of tiles of five holds the mesh:
+      // us per RK step with one / two warps, 64 elements 18.7 / 14.6, 740 18.6
+      // / 14.6, 888 18.6 / 20.7, 1628 20.7 / 28.9.  (A call without elements
+      // primes both forms.)
+      const int sms = s.num_sms > 0 ? s.num_sms : 148;
+      const bool split = s.nelem <= sms * Warp32Plan<TQ, 2>::ELEMS;
+      if (split) {
+        const int rc = launch_warp32<tend_warp32_kernel<TQ, TO, false, 2>, TQ, 2>(s, a, d, m);
+        if (rc != 0 || s.nelem > 0) return rc;
+      }
+      return launch_warp32<tend_warp32_kernel<TQ, TO, false, 1>, TQ, 1>(s, a, d, m);
     }
   }
   // The split-column kernel: orders with one element per tile.
@@ -200,7 +251,7 @@ int run(const LaunchSpec& s) {
   const bool pipe =
       batch || ((s.variant == kVariantPipe || s.variant == kVariantAuto ||
                  s.variant == kVariantSplit || s.variant == kVariantTensor) && can_pipe);
-  if constexpr (!WARP) if (pipe) {
+  if constexpr (!WARP && !(STAGE && kWarp32Kernel<NQ, TC, EXACT>)) if (pipe) {
     const int ntiles =
         batch ? s.batch_ntiles : (s.nelem + PipeGeo<NQ>::EPB - 1) / PipeGeo<NQ>::EPB;
     if (batch)
@@ -281,6 +332,9 @@ int pipe_fits() {
   }
   if constexpr (kWarpKernel<NQ, TC, false>) {
     if (WarpPlan<1>::BYTES <= optin) r |= 4;
+  }
+  if constexpr (STAGE && kWarp32Kernel<NQ, TC, false>) {
+    if (Warp32Plan<TQ, 1>::BYTES <= optin) r |= 4;
   }
   return r;
 }

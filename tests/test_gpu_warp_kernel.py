@@ -1,7 +1,8 @@
-"""The warp-per-element kernel (fast FP64 at p = 7, sdg_tend_warp.cuh) where
-its tiling can go wrong: one element, the element counts around the changes of
-its form (148, 149, 444 and 445 elements on 148 SMs), partial last tiles, halo
-and direct neighbours, and arrays that are not 16-byte aligned."""
+"""The warp-per-element kernels (p = 7: fast FP64, sdg_tend_warp.cuh, and the
+mixed form, sdg_tend_warp32.cuh) where their tiling can go wrong: one element,
+the element counts around the changes of form (148, 149, 444 and 445 elements
+on 148 SMs; mixed 740 and 741), partial last tiles, halo and direct neighbours,
+and arrays that are not 16-byte aligned."""
 import numpy as np
 import pytest
 
@@ -64,5 +65,31 @@ def test_sizes_and_alignment(dims):
     i = b.add(*dims, P, ops, q, u, v, w, dt)
     b.commit()
     b.run(2)
+    assert np.array_equal(b.get(i), single)
+    b.close()
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (5, 3, 1), (37, 20, 1), (19, 39, 1), (149, 11, 1)])
+def test_mixed_sizes(dims):
+    ops = sdg.read_operators(P)
+    mesh = sdg.mesh_setup(*dims, P, ops.x1D)
+    omesh = orc.mesh_setup(*dims, P, ops.x1D)
+    q, u, v, w = sdg.init_fields(mesh, ic_kind=1, seed=9, vel_kind=1)
+    dt = 0.1 / max(dims) / (P + 1) ** 2
+    h = sdg.Handle(ops, mesh, sdg.FLAG_MIXED)
+    h.set_state(q, u, v, w)
+    h.rk3_steps(dt, 3)
+    single = h.get_field()
+    h.close()
+    qo = q.copy(order="F")
+    orc.run_rk3(orc.OPT1, qo, u, v, w, ops, omesh, dt, 3)
+    ref = qo[:, : mesh.Ne]
+    assert np.linalg.norm(single - ref) <= 1e-5 * np.linalg.norm(ref)   # the mixed form's bar
+
+    # The batch always runs one warp per element: the same bits.
+    b = sdg.Batch(sdg.FLAG_MIXED)
+    i = b.add(*dims, P, ops, q, u, v, w, dt)
+    b.commit()
+    b.run(3)
     assert np.array_equal(b.get(i), single)
     b.close()
