@@ -495,10 +495,11 @@ struct Ensemble {
 
   // One RK stage of a group: one batched launch, or one launch per member
   // for the one-tile-per-block variants.
-  int stage(Group* g, int st, cudaStream_t s, int variant) {
+  int stage(Group* g, int st, cudaStream_t s, int variant, bool chained = false) {
     if (g->members.empty()) return SDG_OK;
     LaunchSpec l = spec(g, st, s);
     l.variant = variant;
+    l.pdl = chained;
     if (variant == kVariantPipe || variant == kVariantSplit) {
       l.batch_insts = g->d_insts + st * g->inst_cap;
       l.batch_tiles = g->d_tiles;
@@ -543,7 +544,9 @@ struct Ensemble {
       cudaStream_t gs = concurrent ? g->stream : s;
       if (concurrent) ENS_CUDA(cudaStreamWaitEvent(gs, fork, 0));
       for (int st = 0; st < 3; ++st) {
-        int rc = stage(g, st, gs, g->variant);
+        // Each stage as a programmatic dependent launch on the one before it
+        // (the first, which may follow other work, not).
+        int rc = stage(g, st, gs, g->variant, st > 0);
         if (rc) return rc;
       }
       if (concurrent) {

@@ -273,7 +273,8 @@ struct sdg_handle {
   int red_blocks = 0;
 
   // Step graph.
-  cudaGraphExec_t graph = nullptr;
+  cudaGraphExec_t graph = nullptr;       // of one step of size graph_dt
+  cudaGraphExec_t graph_many = nullptr;  // of kGraphSteps of them
   double graph_dt = 0.0;
   // Graph of an sdg_rk3_steps_host call of host_graph_steps steps (uploads,
   // chunked stages and downloads) for the pinned host array host_graph_q
@@ -300,7 +301,14 @@ struct sdg_handle {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
 
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  bool rk_pending = false;   // ev0/ev1 bracket an unaccounted rk3 batch
+  // Events around the last kRkSpans sdg_rk3_steps calls whose device time is
+  // not in t_rk yet (a call waits for the one kRkSpans before it, no sooner).
+  static constexpr int kRkSpans = 8;
+  struct RkSpan {
+    cudaEvent_t a = nullptr, b = nullptr;
+    bool pending = false;
+  } rk_span[kRkSpans];
+  int rk_next = 0;
   double t_tend = 0, t_rk = 0, t_halo = 0, t_copy = 0;
   long long launches = 0;
 };
@@ -312,6 +320,7 @@ void free_handle(sdg_handle* h) {
   cudaSetDevice(h->dev);
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->graph) cudaGraphExecDestroy(h->graph);
+  if (h->graph_many) cudaGraphExecDestroy(h->graph_many);
   if (h->host_graph) cudaGraphExecDestroy(h->host_graph);
   void* ptrs[] = {h->lift64, h->lift32, h->pb_halo, h->pb_direct, h->esc64,
                   h->esc32,  h->fsc64,  h->fsc32,   h->hsrc,      h->io[0],
@@ -323,6 +332,10 @@ void free_handle(sdg_handle* h) {
     if (p) cudaFree(p);
   if (h->ev0) cudaEventDestroy(h->ev0);
   if (h->ev1) cudaEventDestroy(h->ev1);
+  for (auto& r : h->rk_span) {
+    if (r.a) cudaEventDestroy(r.a);
+    if (r.b) cudaEventDestroy(r.b);
+  }
   for (cudaEvent_t e : h->ev_up) cudaEventDestroy(e);
   for (cudaEvent_t e : h->ev_fin) cudaEventDestroy(e);
   if (h->ev_in) cudaEventDestroy(h->ev_in);
@@ -516,7 +529,7 @@ int ensure_state(sdg_handle* h) {
 // stage 3: q0 <- 1/3 q0 + 2/3 (q2 + dt*L(q2))  (main.f90:58-74 with the
 // coefficients of mod_common.f90:29-30).  The step-start copy q0 = q of
 // main.f90:53-56 disappears: q0 is the step's input buffer.
-int enqueue_stage_range(sdg_handle* h, int st, double dt, int e0, int n) {
+int enqueue_stage_range(sdg_handle* h, int st, double dt, int e0, int n, bool chained = false) {
   const bool f32 = mixed(h);
   const int* pb = h->direct_ok ? h->pb_direct : h->pb_halo;
   const double ra[3] = {0.0, 0.75, 1.0 / 3.0};
@@ -541,6 +554,7 @@ int enqueue_stage_range(sdg_handle* h, int st, double dt, int e0, int n) {
   s.rk_b = rb[st];
   s.dt = dt;
   s.field_maps = h->has_maps ? h->maps[st] : nullptr;
+  s.pdl = chained;
   s.elem0 = e0;
   s.nelem = n;
   return launch_tend(s);
@@ -574,10 +588,12 @@ int prime_stages(sdg_handle* h) {
   return SDG_OK;
 }
 
-// Enqueues one SSP-RK3 step (main.f90:51-74) on the handle's stream.
-int enqueue_step(sdg_handle* h, double dt) {
+// Enqueues one SSP-RK3 step (main.f90:51-74) on the handle's stream; with
+// `chained`, stage kernels as programmatic dependent launches: each starts
+// (operators, velocities) while the one before it ends.
+int enqueue_step(sdg_handle* h, double dt, bool chained) {
   for (int st = 0; st < 3; ++st) {
-    int rc = enqueue_stage(h, st, dt);
+    int rc = enqueue_stage_range(h, st, dt, 0, h->Ne, chained);
     if (rc) return rc;
   }
   return SDG_OK;
@@ -589,45 +605,82 @@ int check_handle(sdg_handle* h) {
   return SDG_OK;
 }
 
-// Adds the device time of the last rk3 batch to its timer once the stream
-// has passed it.
-void account_rk(sdg_handle* h) {
-  if (!h->rk_pending) return;
+// Adds the device time of an sdg_rk3_steps call to its timer once the stream
+// has passed it; of every pending one.
+void account_span(sdg_handle* h, sdg_handle::RkSpan* r) {
+  if (!r->pending) return;
   float ms = 0;
-  if (cudaEventSynchronize(h->ev1) == cudaSuccess &&
-      cudaEventElapsedTime(&ms, h->ev0, h->ev1) == cudaSuccess)
+  if (cudaEventSynchronize(r->b) == cudaSuccess &&
+      cudaEventElapsedTime(&ms, r->a, r->b) == cudaSuccess)
     h->t_rk += 1e-3 * ms;
-  h->rk_pending = false;
+  r->pending = false;
 }
 
-// The CUDA graph of one RK3 step of size dt (captured on first use).
-int ensure_graph(sdg_handle* h, double dt) {
-  if (h->graph && h->graph_dt == dt) return SDG_OK;
-  if (h->graph) {
-    cudaGraphExecDestroy(h->graph);
-    h->graph = nullptr;
-  }
+void account_rk(sdg_handle* h) {
+  for (auto& r : h->rk_span) account_span(h, &r);
+}
+
+// Steps of the longer step graph.  Launching one graph after another leaves a
+// gap that a small mesh feels, and only the kernels inside a graph overlap
+// their ends.  Measured, us per step with 1 / 2 / 4 / 8 / 16 steps a graph
+// (before the chained launches): 64 elements exact p = 7 14.4 / 12.3 / 11.8 /
+// 11.5 / 11.5, 512 elements exact p = 3 10.8 / 10.3 / 9.8 / 9.5 / 9.2; with
+// them and 8 steps a graph 10.8 and 8.8.
+constexpr int kGraphSteps = 8;
+// Calls of fewer steps take the one-step graph alone: capturing the longer one
+// costs about as much as it gives there.
+constexpr int kGraphManyFrom = 24;
+
+int capture_steps(sdg_handle* h, double dt, int steps, cudaGraphExec_t* out) {
   cudaGraph_t g;
   SDG_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = enqueue_step(h, dt);
+  int rc = SDG_OK;
+  for (int i = 0; i < steps && !rc; ++i) rc = enqueue_step(h, dt, true);
   cudaError_t ee = cudaStreamEndCapture(h->stream, &g);
   if (ee == cudaSuccess && rc) cudaGraphDestroy(g);
   if (rc) return rc;
   if (ee != cudaSuccess)
     return fail(SDG_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(ee));
-  ee = cudaGraphInstantiate(&h->graph, g, 0);
+  ee = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
-  if (ee != cudaSuccess)
+  if (ee != cudaSuccess) {
+    *out = nullptr;
     return fail(SDG_ERR_CUDA, "graph instantiate failed: %s", cudaGetErrorString(ee));
-  h->graph_dt = dt;
+  }
+  return SDG_OK;
+}
+
+// The CUDA graphs of RK3 steps of size dt that a call of nsteps takes
+// (captured on first use).
+int ensure_graph(sdg_handle* h, double dt, int nsteps) {
+  if (h->graph_dt != dt) {
+    if (h->graph) cudaGraphExecDestroy(h->graph);
+    if (h->graph_many) cudaGraphExecDestroy(h->graph_many);
+    h->graph = h->graph_many = nullptr;
+    h->graph_dt = dt;
+  }
+  int rc = SDG_OK;
+  if (!h->graph && (rc = capture_steps(h, dt, 1, &h->graph))) return rc;
+  if (nsteps >= kGraphManyFrom && !h->graph_many)
+    rc = capture_steps(h, dt, kGraphSteps, &h->graph_many);
+  return rc;
+}
+
+// Enqueues nsteps RK3 steps through the step graphs.
+int launch_steps(sdg_handle* h, int nsteps) {
+  for (; nsteps >= kGraphSteps && h->graph_many; nsteps -= kGraphSteps)
+    SDG_CUDA(cudaGraphLaunch(h->graph_many, h->stream));
+  for (; nsteps > 0; --nsteps) SDG_CUDA(cudaGraphLaunch(h->graph, h->stream));
   return SDG_OK;
 }
 
 // Releases the graphs (they hold kernel arguments: variant, test hooks).
 void drop_graphs(sdg_handle* h) {
   if (h->graph) cudaGraphExecDestroy(h->graph);
+  if (h->graph_many) cudaGraphExecDestroy(h->graph_many);
   if (h->host_graph) cudaGraphExecDestroy(h->host_graph);
   h->graph = nullptr;
+  h->graph_many = nullptr;
   h->host_graph = nullptr;
   h->host_graph_q = nullptr;
 }
@@ -974,9 +1027,7 @@ int enqueue_host_steps(sdg_handle* h, double* q, double dt, int nsteps) {
     rc = enqueue_steps_chunked(h, dt, nsteps, true, q);
   } else {
     rc = enqueue_steps_chunked(h, dt, 1, true, nullptr);
-    for (int i = 0; i < nsteps - 2 && !rc; ++i)
-      if (cudaGraphLaunch(h->graph, h->stream) != cudaSuccess)
-        rc = fail(SDG_ERR_CUDA, "graph launch failed");
+    if (!rc) rc = launch_steps(h, nsteps - 2);
     h->launches += 3LL * (nsteps - 2);
     if (!rc) rc = enqueue_steps_chunked(h, dt, 1, false, q);
   }
@@ -1282,12 +1333,18 @@ int sdg_rk3_steps(sdg_handle* h, double dt, int nsteps) {
                 "stages; run sdg_update_halo_stage, the exchange and sdg_rk3_stage");
   if (nsteps == 0) return SDG_OK;
   if ((rc = prime_stages(h))) return rc;
-  if ((rc = ensure_graph(h, dt))) return rc;
-  account_rk(h);
-  SDG_CUDA(cudaEventRecord(h->ev0, h->stream));
-  for (int i = 0; i < nsteps; ++i) SDG_CUDA(cudaGraphLaunch(h->graph, h->stream));
-  SDG_CUDA(cudaEventRecord(h->ev1, h->stream));
-  h->rk_pending = true;
+  if ((rc = ensure_graph(h, dt, nsteps))) return rc;
+  sdg_handle::RkSpan* span = &h->rk_span[h->rk_next];
+  h->rk_next = (h->rk_next + 1) % sdg_handle::kRkSpans;
+  account_span(h, span);
+  if (!span->b) {
+    SDG_CUDA(cudaEventCreate(&span->a));
+    SDG_CUDA(cudaEventCreate(&span->b));
+  }
+  SDG_CUDA(cudaEventRecord(span->a, h->stream));
+  if ((rc = launch_steps(h, nsteps))) return rc;
+  SDG_CUDA(cudaEventRecord(span->b, h->stream));
+  span->pending = true;
   h->launches += 3LL * nsteps;
   return SDG_OK;
 }
@@ -1310,7 +1367,7 @@ int sdg_rk3_steps_host(sdg_handle* h, double* q, double dt, int nsteps) {
     return sdg_get_field(h, SDG_FIELD_Q, q);
   }
   if ((rc = prime_stages(h))) return rc;
-  if (nsteps > kPlanSteps && (rc = ensure_graph(h, dt))) return rc;
+  if (nsteps > kPlanSteps && (rc = ensure_graph(h, dt, nsteps))) return rc;
   account_rk(h);
   h->have_q = true;
   const size_t NE = static_cast<size_t>(h->Np) * h->Ne;

@@ -88,6 +88,9 @@ struct LaunchSpec {
   unsigned wait_spins; // spin limit of a bounded wait; 0: the default
   int inject_skip;     // test hook: tile + 1 whose copies are skipped; 0: none
   int num_sms;         // multiprocessors of the device
+  // Programmatic dependent launch on the launch before it in the stream, which
+  // must be a stage kernel too (or wait for nothing that stages write).
+  bool pdl;
   // Batched launch (pipelined kernel only): device arrays of BatchInst and
   // BatchTile (sdg_tend.cuh) and the tile count; null for one instance.
   const void* batch_insts;

@@ -22,6 +22,24 @@ namespace {
 
 constexpr int NQ = SDG_NQ;
 
+// kern<<<grid, threads, smem, s.stream>>>(args...), as a programmatic dependent
+// launch where the spec asks for one.
+template <typename... KArgs, typename... Args>
+int launch_kernel(void (*kern)(KArgs...), int grid, int threads, size_t smem,
+                  const LaunchSpec& s, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s.stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = s.pdl && kPdl<NQ> ? 1 : 0;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, args...));
+}
+
 // Launches a persistent pipelined kernel: attribute and occupancy set-up on
 // the first call of each instantiation (a call with no tiles only primes
 // it, e.g. before a stream capture), then one block per resident slot.  The
@@ -52,8 +70,7 @@ int launch_pipe(size_t smem, int ntiles, const LaunchSpec& s, const Args& a, con
   }
   if (ntiles <= 0) return 0;
   const int grid = std::min(ntiles, blocks_per_sm * (s.num_sms > 0 ? s.num_sms : 148));
-  kern<<<grid, THREADS, smem, s.stream>>>(a, d);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, grid, THREADS, smem, s, a, d);
 }
 
 // Launches the warp-per-element kernel: one block per SM, or one per tile
@@ -73,8 +90,7 @@ int launch_warp(int ntiles, const LaunchSpec& s, const Args& a, const Dm& d) {
   }
   if (ntiles <= 0) return 0;
   const int grid = std::min(ntiles, s.num_sms > 0 ? s.num_sms : 148);
-  kern<<<grid, WarpPlan<H>::THREADS, WarpPlan<H>::BYTES, s.stream>>>(a, d);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, grid, WarpPlan<H>::THREADS, WarpPlan<H>::BYTES, s, a, d);
 }
 
 // The mixed form's warp-per-element kernel: tiles of the most elements a slot
@@ -98,8 +114,7 @@ int launch_warp32(const LaunchSpec& s, Args& a, const Dm& d, const FieldMaps& m)
   const int ntiles = s.batch_tiles ? s.batch_ntiles
                                    : (s.nelem + a.tile_elems - 1) / a.tile_elems;
   if (ntiles <= 0) return 0;
-  kern<<<std::min(ntiles, sms), P::THREADS, P::BYTES, s.stream>>>(a, d, m);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, std::min(ntiles, sms), P::THREADS, P::BYTES, s, a, d, m);
 }
 
 // Warps per element of the warp-per-element kernel for a mesh of `per_sm`
@@ -143,6 +158,7 @@ int run(const LaunchSpec& s) {
   for (int i = 0; i < NQ * NQ; ++i) d.d[i] = static_cast<TC>(s.D[i]);
   for (int i = 0; i < 2 * NQ; ++i) {
     d.lz[i] = s.lift_z ? static_cast<TC>(s.lift_z[i]) : TC(0);
+    if constexpr (!DMat<NQ, TC>::XY) continue;
     d.lx[i] = s.lift_z ? static_cast<TC>(s.lift_z[2 * NQ + i]) : TC(0);
     d.ly[i] = s.lift_z ? static_cast<TC>(s.lift_z[4 * NQ + i]) : TC(0);
   }
@@ -307,8 +323,7 @@ int run(const LaunchSpec& s) {
   if (s.nelem <= 0) return 0;
   a.prefetch_dist = resident * (s.num_sms > 0 ? s.num_sms : 148);
   const int blocks = (s.nelem + G::EPB - 1) / G::EPB;
-  kern<<<blocks, G::THREADS, smem, s.stream>>>(a, d);
-  return static_cast<int>(cudaGetLastError());
+  return launch_kernel(kern, blocks, G::THREADS, smem, s, a, d);
 }
 
 }  // namespace

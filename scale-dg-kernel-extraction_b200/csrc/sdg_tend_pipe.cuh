@@ -529,6 +529,7 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
   static_assert(!(NQ == 8 && sizeof(TC) == 8 && !EXACT),
                 "fast FP64 at Nq = 8: tend_warp_kernel");
 
+  if constexpr (kPdl<NQ>) pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* slots = smem_raw;
   TC* sL = reinterpret_cast<TC*>(smem_raw + NS * P::SLOT + P::FACE);
@@ -559,8 +560,9 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
   // FP32: [4][NQ2] (q, un) pairs of the four faces, face-major.
   V2* fM = reinterpret_cast<V2*>(fa);
 
-  // Producer: one thread fills ring slot `slot` with tile `tile`.
-  auto issue = [&](int tile, int slot) {
+  // Producer: one thread fills ring slot `slot` with tile `tile`: what no stage
+  // writes (parts & 1), then q and q0 (parts & 2).
+  auto issue = [&](int tile, int slot, int parts) {
     // Test hook (host-set): leave this tile's slot empty, so that its wait
     // runs out and the timeout path below is taken.
     if (tile + 1 == A.inject_skip) return;
@@ -583,18 +585,33 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
     size_t plo = 0;
     uint32_t pby = 0, psh = 0;
     if constexpr (RCTX) {
-      *reinterpret_cast<Ctx*>(base + P::OFF_C) = c;
+      if (parts & 1) *reinterpret_cast<Ctx*>(base + P::OFF_C) = c;
       tile_range(c.e0, c.n, sizeof(int) * 6, &plo, &pby, &psh);
       total += pby;
     }
-    mbar_arrive_expect_tx(&bars[slot], total);
+    if constexpr (!kPdl<NQ>) {
+      mbar_arrive_expect_tx(&bars[slot], total);
 #pragma unroll
-    for (int k = 0; k < 6; ++k)
-      bulk_g2s(base + off[k], static_cast<const unsigned char*>(src[k]) + lo[k], by[k],
-               &bars[slot]);
-    if constexpr (RCTX)
-      bulk_g2s(base + P::OFF_P, reinterpret_cast<const unsigned char*>(c.pbase) + plo, pby,
-               &bars[slot]);
+      for (int k = 0; k < 6; ++k)
+        bulk_g2s(base + off[k], static_cast<const unsigned char*>(src[k]) + lo[k], by[k],
+                 &bars[slot]);
+      if constexpr (RCTX)
+        bulk_g2s(base + P::OFF_P, reinterpret_cast<const unsigned char*>(c.pbase) + plo, pby,
+                 &bars[slot]);
+    } else {
+      if (parts & 1) {
+        mbar_arrive_expect_tx(&bars[slot], total);
+#pragma unroll
+        for (int k = 1; k < 6; ++k)
+          bulk_g2s(base + off[k], static_cast<const unsigned char*>(src[k]) + lo[k], by[k],
+                   &bars[slot]);
+        if constexpr (RCTX)
+          bulk_g2s(base + P::OFF_P, reinterpret_cast<const unsigned char*>(c.pbase) + plo, pby,
+                   &bars[slot]);
+      }
+      if (!(parts & 2)) return;
+      bulk_g2s(base, static_cast<const unsigned char*>(src[0]) + lo[0], by[0], &bars[slot]);
+    }
     // q0 (RK stages 2-3) is read by the epilogue straight from global
     // memory; bring the tile's range into L2 now.
     if (STAGE && A.rk_a != 0.0) {
@@ -638,10 +655,16 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
     tc::fence_after_sync();
     tmem = *tmem_slot;
   }
+  if (kPdl<NQ> && threadIdx.x == 0)
+    for (int k = 0; k < NS; ++k) {
+      const int tile = blockIdx.x + k * gridDim.x;
+      if (tile < ntiles) issue(tile, k, 1);
+    }
+  if constexpr (kPdl<NQ>) pdl_wait();
   if (threadIdx.x == 0)
     for (int k = 0; k < NS; ++k) {
       const int tile = blockIdx.x + k * gridDim.x;
-      if (tile < ntiles) issue(tile, k);
+      if (tile < ntiles) issue(tile, k, kPdl<NQ> ? 2 : 3);
     }
 
   for (int it = 0;; ++it) {
@@ -700,7 +723,7 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
     // slot is free: refill it with the tile NS iterations on from it.
     if (threadIdx.x == 0 && it > 0) {
       const int nt = blockIdx.x + (it - 1 + NS) * gridDim.x;
-      if (nt < ntiles) issue(nt, (it - 1) % NS);
+      if (nt < ntiles) issue(nt, (it - 1) % NS, 3);
     }
 
     unsigned char* sb = slots + slot * P::SLOT;

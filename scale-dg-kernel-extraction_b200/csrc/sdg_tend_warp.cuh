@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
   constexpr size_t EB = NP * sizeof(double);  // bytes of an element's field
   constexpr int NS = VEC ? P::NSTAGE : 1;
   constexpr unsigned kAll = 0xffffffffu;
+  pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + P::NSTAGE * P::SLOT + P::EXCH);
   uint64_t* empty = full + P::NSTAGE;
@@ -159,9 +160,37 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     }
     __syncthreads();
   }
+  // Copies of tile `tile` into slot `slot`: the velocities (parts & 1), then q
+  // with the prefetch of q0 (parts & 2).
+  auto copy = [&](int tile, int slot, int parts) {
+    const Ctx t = context(tile);
+    const size_t off = static_cast<size_t>(t.e0) * EB;
+    const uint32_t bytes = static_cast<uint32_t>(t.n * EB);
+    unsigned char* dst = smem_raw + slot * P::SLOT;
+    const void* src[4] = {t.q, t.u, t.v, t.w};
+    if (parts & 1) {
+      mbar_arrive_expect_tx(&full[slot], 4 * bytes);
+#pragma unroll
+      for (int k = 1; k < 4; ++k)
+        bulk_g2s(dst + k * P::FIELD, static_cast<const unsigned char*>(src[k]) + off, bytes,
+                 &full[slot]);
+    }
+    if (!(parts & 2)) return;
+    bulk_g2s(dst, static_cast<const unsigned char*>(src[0]) + off, bytes, &full[slot]);
+    if (STAGE && A.rk_a != 0.0)
+      bulk_prefetch_l2(reinterpret_cast<const unsigned char*>(t.q0) + off, bytes);
+  };
   if (warp == P::WARPS) {
     // Producer: fills slot it % NS with this block's tile it once the seven
     // warps are done with tile it - NS.
+    // The first tiles' velocities go before the wait for the previous stage.
+    int ahead = 0;
+    for (; VEC && lane == 0 && ahead < NS; ++ahead) {
+      const int tile = blockIdx.x + ahead * gridDim.x;
+      if (tile >= ntiles || tile + 1 == A.inject_skip) break;
+      copy(tile, ahead, 1);
+    }
+    pdl_wait();
     for (int it = 0; VEC && lane == 0; ++it) {
       const int tile = blockIdx.x + it * gridDim.x;
       if (tile >= ntiles) break;
@@ -171,18 +200,7 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
         break;  // the consumers wait for what is in flight
       }
       if (tile + 1 == A.inject_skip) continue;  // test hook: leave the slot empty
-      const Ctx t = context(tile);
-      const size_t off = static_cast<size_t>(t.e0) * EB;
-      const uint32_t bytes = static_cast<uint32_t>(t.n * EB);
-      unsigned char* dst = smem_raw + slot * P::SLOT;
-      mbar_arrive_expect_tx(&full[slot], 4 * bytes);
-      const void* src[4] = {t.q, t.u, t.v, t.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        bulk_g2s(dst + k * P::FIELD, static_cast<const unsigned char*>(src[k]) + off, bytes,
-                 &full[slot]);
-      if (STAGE && A.rk_a != 0.0)
-        bulk_prefetch_l2(reinterpret_cast<const unsigned char*>(t.q0) + off, bytes);
+      copy(tile, slot, it < ahead ? 2 : 3);
     }
     return;
   }
@@ -264,6 +282,7 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     int row = 0;
     const Ctx t = context(blockIdx.x);
     load_row(t, &row, &met);
+    pdl_wait();
     gather(t, row);
     gather_z(t, row);
   }
