@@ -155,8 +155,8 @@ struct Group {
   int flags = 0;
   Ops* ops = nullptr;
   std::vector<Inst*> members;
-  int epb = 1;
   bool warp = false;            // the warp-per-element kernel runs it
+  bool line = false;            // the line kernel is built for it
   int variant = kVariantAuto;   // set by the autotuner
   bool dirty = true;
   // Device tables, two buffers: a rebuild writes the buffer that no launch
@@ -283,13 +283,13 @@ struct Ensemble {
     g->ops = o;
     // The fast pipelined kernels need the factored lift.
     const bool exact = !mixed && (flags & SDG_FLAG_EXACT);
-    g->epb = batch_elems_per_tile(nq, mixed, exact, !o->lift_z.empty());
     g->warp = warp_kernel(nq, mixed, exact, !o->lift_z.empty());
+    g->line = !g->warp && line_kernel(nq, mixed, exact, !o->lift_z.empty());
     const bool can_pipe = pipe_supported(nq, mixed ? kStageMixed2 : kStageF64) &&
                           pipe_supported(nq, mixed ? kStageMixed1 : kStageF64) &&
                           pipe_supported(nq, mixed ? kStageMixed3 : kStageF64) &&
                           (exact || !o->lift_z.empty());
-    g->variant = can_pipe ? kVariantPipe : kVariantBlock;
+    g->variant = g->line ? kVariantLine : can_pipe ? kVariantPipe : kVariantBlock;
     ENS_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
     ENS_CUDA(cudaEventCreateWithFlags(&g->done, cudaEventDisableTiming));
     *out = g.get();
@@ -384,10 +384,11 @@ struct Ensemble {
     const int ni = static_cast<int>(g->members.size());
     g->h_insts.assign(3L * std::max(ni, 1), BatchInst{});
     g->h_tiles.clear();
-    // The warp-per-element kernel takes shorter tiles as well: a small group
-    // spreads over the SMs.
-    int epb = g->epb;
-    if (g->warp) {
+    // The warp-per-element and line kernels take shorter tiles as well: a small
+    // group spreads over the SMs.
+    const bool exact = !g->mixed && (g->flags & SDG_FLAG_EXACT);
+    int epb = batch_elems_per_tile(g->nq, g->mixed, exact, !g->ops->lift_z.empty(), g->variant);
+    if (g->warp || g->variant == kVariantLine) {
       long total = 0;
       for (Inst* I : g->members) total += I->ne;
       epb = static_cast<int>(std::max(1L, std::min<long>(epb, (total + num_sms - 1) / num_sms)));
@@ -500,7 +501,7 @@ struct Ensemble {
     LaunchSpec l = spec(g, st, s);
     l.variant = variant;
     l.pdl = chained;
-    if (variant == kVariantPipe || variant == kVariantSplit) {
+    if (variant == kVariantPipe || variant == kVariantSplit || variant == kVariantLine) {
       l.batch_insts = g->d_insts + st * g->inst_cap;
       l.batch_tiles = g->d_tiles;
       l.batch_ntiles = g->ntiles;
@@ -565,6 +566,7 @@ struct Ensemble {
     std::vector<int> cands;
     // One kernel whatever the variant: launched as the pipelined one.
     if (g->warp) return {kVariantPipe};
+    if (g->line) cands.push_back(kVariantLine);
     const bool can_pipe = pipe_supported(g->nq, g->mixed ? kStageMixed2 : kStageF64) &&
                           pipe_supported(g->nq, g->mixed ? kStageMixed1 : kStageF64) &&
                           pipe_supported(g->nq, g->mixed ? kStageMixed3 : kStageF64);
@@ -593,7 +595,10 @@ struct Ensemble {
     for (auto& kvp : groups) {
       Group* g = kvp.second.get();
       const std::vector<int> c = candidates(g);
-      if (std::find(c.begin(), c.end(), v) != c.end()) g->variant = v;
+      if (std::find(c.begin(), c.end(), v) != c.end()) {
+        g->variant = v;
+        g->dirty = true;
+      }
     }
   }
 
@@ -610,6 +615,10 @@ struct Ensemble {
       double best = 1e30;
       int best_v = cands[0];
       for (int v : cands) {
+        // The tile table is the variant's own.
+        g->variant = v;
+        g->dirty = true;
+        if ((rc = rebuild(g))) return rc;
         for (int w = 0; w < 2; ++w)
           if ((rc = stage(g, 1, g->stream, v))) return rc;
         ENS_CUDA(cudaEventRecord(e0, g->stream));
@@ -629,6 +638,7 @@ struct Ensemble {
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
       g->variant = best_v;
+      g->dirty = true;
     }
     return check_status();
   }
@@ -644,7 +654,8 @@ struct Ensemble {
       for (int st = 0; st < 3; ++st) {
         LaunchSpec l = spec(g, st, g->stream);
         l.variant = g->variant;
-        if (g->variant == kVariantPipe || g->variant == kVariantSplit) {
+        if (g->variant == kVariantPipe || g->variant == kVariantSplit ||
+            g->variant == kVariantLine) {
           l.batch_insts = g->d_insts;
           l.batch_tiles = g->d_tiles;
           l.batch_ntiles = 0;

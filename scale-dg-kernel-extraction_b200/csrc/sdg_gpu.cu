@@ -69,10 +69,17 @@ int encode_field_map(void* map, const void* base, int elem_bytes, long nelem) {
   return SDG_OK;
 }
 
-int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored) {
+bool line_kernel(int nq, bool mixed, bool exact, bool factored) {
   int epb = 1;
-  pipe_info(nq, kTendF64, &epb);
-  return warp_kernel(nq, mixed, exact, factored) ? (mixed ? kWarpElems32 : kWarpElems) : epb;
+  return (exact || factored) &&
+         (pipe_info(nq, mixed ? kStageMixed1 : kStageF64, &epb) & (exact ? 16 : 8)) != 0;
+}
+
+int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored, int variant) {
+  int epb = 1;
+  const int info = pipe_info(nq, mixed ? kStageMixed1 : kStageF64, &epb);
+  if (warp_kernel(nq, mixed, exact, factored)) return mixed ? kWarpElems32 : kWarpElems;
+  return variant == kVariantLine ? info >> 8 : epb;
 }
 
 bool pipe_supported(int nq, int kind) {

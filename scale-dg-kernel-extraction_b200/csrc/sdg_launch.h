@@ -98,9 +98,13 @@ struct LaunchSpec {
   int batch_ntiles;
 };
 
-// Elements per tile of the batched kernels for a given order and form (the
-// tile size a batch's tile table must use); `factored`: Lift_mat factorises.
-int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored);
+// Elements per tile of the batched kernel of `variant` for a given order and
+// form (the tile size a batch's tile table must use); `factored`: Lift_mat
+// factorises.
+int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored, int variant);
+
+// Whether the line kernel (sdg_tend_line.cuh) is built for this order and form.
+bool line_kernel(int nq, bool mixed, bool exact, bool factored);
 
 // Whether the fast FP64 or mixed form of this order runs a warp-per-element
 // kernel (sdg_tend_warp.cuh, sdg_tend_warp32.cuh), whatever variant is asked
@@ -148,7 +152,8 @@ enum KernelVariant {
   kVariantPipe = 2,
   kVariantBlockOcc = 3,
   kVariantSplit = 4,
-  kVariantTensor = 5
+  kVariantTensor = 5,
+  kVariantLine = 6  // tend_line_kernel: chosen by Auto and by the batch, never asked for
 };
 
 // Returns 0 when launched, -1 when this unit does not hold spec.nq,

@@ -142,12 +142,10 @@ struct SmemLayout {
 template <int NQ, typename TC>
 struct DMat {
   TC d[NQ * NQ];
-  // Lift factors of the factored fast lift, faces (-z, +z) and, where a kernel
-  // takes them from here, (-x, +x), (-y, +y).
-  static constexpr bool XY = NQ == 8;
+  // Lift factors of the factored fast lift, faces (-z, +z), (-x, +x), (-y, +y).
   TC lz[2 * NQ];
-  TC lx[XY ? 2 * NQ : 1];
-  TC ly[XY ? 2 * NQ : 1];
+  TC lx[2 * NQ];
+  TC ly[2 * NQ];
 };
 
 // Sum_{l} A(l)*B(l) in the reference's order (see header comment).
@@ -324,7 +322,7 @@ struct TendArgs {
   // One-tile-per-block kernel: block b prefetches into L2 the inputs of
   // block b + prefetch_dist (about one resident wave ahead); 0 disables.
   int prefetch_dist;
-  // Warp-per-element kernel: elements per tile of a single instance (1..7).
+  // Warp-per-element and line kernels: elements per tile of a single instance.
   int tile_elems;
   // Batched launches (pipelined kernel only): per-instance arrays and a
   // table of element tiles.  Null for a single instance, whose tiles are

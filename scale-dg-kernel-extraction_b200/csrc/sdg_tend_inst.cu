@@ -10,6 +10,7 @@
 #include "sdg_tend.cuh"
 #include "sdg_tend_pipe.cuh"
 #include "sdg_tend_split.cuh"
+#include "sdg_tend_line.cuh"
 #include "sdg_tend_warp.cuh"
 #include "sdg_tend_warp32.cuh"
 
@@ -23,10 +24,10 @@ namespace {
 constexpr int NQ = SDG_NQ;
 
 // kern<<<grid, threads, smem, s.stream>>>(args...), as a programmatic dependent
-// launch where the spec asks for one.
+// launch where the spec asks for one and the kernel takes part.
 template <typename... KArgs, typename... Args>
 int launch_kernel(void (*kern)(KArgs...), int grid, int threads, size_t smem,
-                  const LaunchSpec& s, const Args&... args) {
+                  const LaunchSpec& s, bool pdl, const Args&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(threads);
@@ -36,7 +37,7 @@ int launch_kernel(void (*kern)(KArgs...), int grid, int threads, size_t smem,
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = s.pdl && kPdl<NQ> ? 1 : 0;
+  cfg.numAttrs = s.pdl && pdl ? 1 : 0;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, args...));
 }
 
@@ -51,7 +52,7 @@ int launch_kernel(void (*kern)(KArgs...), int grid, int threads, size_t smem,
 // whose shared memory, registers and 32 TMEM columns allow more).
 template <auto KERN, int THREADS = PipeGeo<NQ>::THREADS, typename Args, typename Dm>
 int launch_pipe(size_t smem, int ntiles, const LaunchSpec& s, const Args& a, const Dm& d,
-                int floor_blocks = 0) {
+                int floor_blocks = 0, bool pdl = kPdl<NQ>) {
   constexpr auto kern = KERN;
   static DeviceSetup setup;  // blocks per SM, per kernel and device
   const int dev = setup_device();
@@ -70,7 +71,7 @@ int launch_pipe(size_t smem, int ntiles, const LaunchSpec& s, const Args& a, con
   }
   if (ntiles <= 0) return 0;
   const int grid = std::min(ntiles, blocks_per_sm * (s.num_sms > 0 ? s.num_sms : 148));
-  return launch_kernel(kern, grid, THREADS, smem, s, a, d);
+  return launch_kernel(kern, grid, THREADS, smem, s, pdl, a, d);
 }
 
 // Launches the warp-per-element kernel: one block per SM, or one per tile
@@ -90,7 +91,7 @@ int launch_warp(int ntiles, const LaunchSpec& s, const Args& a, const Dm& d) {
   }
   if (ntiles <= 0) return 0;
   const int grid = std::min(ntiles, s.num_sms > 0 ? s.num_sms : 148);
-  return launch_kernel(kern, grid, WarpPlan<H>::THREADS, WarpPlan<H>::BYTES, s, a, d);
+  return launch_kernel(kern, grid, WarpPlan<H>::THREADS, WarpPlan<H>::BYTES, s, true, a, d);
 }
 
 // The mixed form's warp-per-element kernel: tiles of the most elements a slot
@@ -114,7 +115,7 @@ int launch_warp32(const LaunchSpec& s, Args& a, const Dm& d, const FieldMaps& m)
   const int ntiles = s.batch_tiles ? s.batch_ntiles
                                    : (s.nelem + a.tile_elems - 1) / a.tile_elems;
   if (ntiles <= 0) return 0;
-  return launch_kernel(kern, std::min(ntiles, sms), P::THREADS, P::BYTES, s, a, d, m);
+  return launch_kernel(kern, std::min(ntiles, sms), P::THREADS, P::BYTES, s, true, a, d, m);
 }
 
 // Warps per element of the warp-per-element kernel for a mesh of `per_sm`
@@ -158,7 +159,6 @@ int run(const LaunchSpec& s) {
   for (int i = 0; i < NQ * NQ; ++i) d.d[i] = static_cast<TC>(s.D[i]);
   for (int i = 0; i < 2 * NQ; ++i) {
     d.lz[i] = s.lift_z ? static_cast<TC>(s.lift_z[i]) : TC(0);
-    if constexpr (!DMat<NQ, TC>::XY) continue;
     d.lx[i] = s.lift_z ? static_cast<TC>(s.lift_z[2 * NQ + i]) : TC(0);
     d.ly[i] = s.lift_z ? static_cast<TC>(s.lift_z[4 * NQ + i]) : TC(0);
   }
@@ -222,6 +222,32 @@ int run(const LaunchSpec& s) {
         if (rc != 0 || s.nelem > 0) return rc;
       }
       return launch_warp32<tend_warp32_kernel<TQ, TO, false, 1>, TQ, 1>(s, a, d, m);
+    }
+  }
+  // The line kernel.
+  if constexpr (kLineAuto<NQ, TC, EXACT> && !WARP && !(STAGE && kWarp32Kernel<NQ, TC, EXACT>)) {
+    using LP = LinePlan<NQ, TQ, TV, TC>;
+    static_assert(LP::BYTES <= kPipeMaxSmem, "line kernel: shared memory");
+    const bool can = LP::BYTES <= device_smem_optin() && (EXACT || s.lift_z != nullptr) &&
+                     (batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) && aligned(s.w) &&
+                                aligned(s.escale) && aligned(s.fscale) && aligned(s.pbase) &&
+                                (s.q0 == nullptr || aligned(s.q0))));
+    // Small meshes stay with the kernels before it at Nq = 16 (which run two
+    // blocks per SM: 216 elements 48 against 62 us a step, 512 112 against 122)
+    // and in the exact forms (which wait for the lift table's loads one by one:
+    // p = 11, 64 elements 25.4 against 27.1, 343 elements 61.5 against 53.9).
+    const bool few = (NQ == 16 || EXACT) && !batch && s.nelem > 0 &&
+                     s.nelem <= (EXACT ? 2 : 4) * (s.num_sms > 0 ? s.num_sms : 148);
+    if (can && !few && (s.variant == kVariantLine || (s.variant == kVariantAuto && !batch))) {
+      // Shorter tiles where the longest would leave a block without one.
+      const int slots = LineTile<NQ, TC>::BLOCKS * (s.num_sms > 0 ? s.num_sms : 148);
+      a.tile_elems = std::max(1, std::min(LP::E, (s.nelem + slots - 1) / slots));
+      const int ntiles = batch ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
+      if (batch)
+        return launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, true>,
+                           LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);
+      return launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, false>,
+                         LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);
     }
   }
   // The split-column kernel: orders with one element per tile.
@@ -323,7 +349,7 @@ int run(const LaunchSpec& s) {
   if (s.nelem <= 0) return 0;
   a.prefetch_dist = resident * (s.num_sms > 0 ? s.num_sms : 148);
   const int blocks = (s.nelem + G::EPB - 1) / G::EPB;
-  return launch_kernel(kern, blocks, G::THREADS, smem, s, a, d);
+  return launch_kernel(kern, blocks, G::THREADS, smem, s, kPdl<NQ>, a, d);
 }
 
 }  // namespace
@@ -334,7 +360,8 @@ int run(const LaunchSpec& s) {
 // Which persistent plans fit both the build's limit and the current
 // device's per-block opt-in: bit 0 the pipelined kernel, bit 1 the
 // split-column kernel (orders with one element per tile), bit 2 the
-// warp-per-element kernel of the fast FP64 form.
+// warp-per-element kernel of the fast FP64 form, bits 3 and 4 the line kernel
+// of the fast and the exact forms with its elements per tile from bit 8 up.
 template <typename TQ, typename TV, typename TC, bool STAGE>
 int pipe_fits() {
   const size_t optin = device_smem_optin();
@@ -350,6 +377,11 @@ int pipe_fits() {
   }
   if constexpr (STAGE && kWarp32Kernel<NQ, TC, false>) {
     if (Warp32Plan<TQ, 1>::BYTES <= optin) r |= 4;
+  }
+  if constexpr (kLineAuto<NQ, TC, false> || kLineAuto<NQ, TC, true>) {
+    if (LinePlan<NQ, TQ, TV, TC>::BYTES <= optin)
+      r |= (kLineAuto<NQ, TC, false> ? 8 : 0) | (kLineAuto<NQ, TC, true> ? 16 : 0) |
+           LineTile<NQ, TC>::E << 8;
   }
   return r;
 }
