@@ -67,7 +67,8 @@ struct Warp32Plan {
   static constexpr int THREADS = 32 * (WARPS + 1);
   static constexpr size_t SLOT = ELEMS * ELEM;
   // The swizzle acts on address bits: slots start at 1024-byte boundaries.
-  static constexpr size_t BYTES = NSTAGE * SLOT + 16 * NSTAGE + 1024;
+  static constexpr size_t OFF_C = NSTAGE * SLOT + 16 * NSTAGE;
+  static constexpr size_t BYTES = OFF_C + 4 * 128 + 1024;  // contexts as in WarpPlan
 };
 static_assert(Warp32Plan<float, 1>::BYTES <= kPipeMaxSmem &&
                   Warp32Plan<double, 1>::BYTES <= kPipeMaxSmem,
@@ -192,11 +193,22 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     fence_barrier_init();
   }
   __syncthreads();
+  // Contexts of the block's tiles, as in tend_warp_kernel (batched launches).
+  static_assert(sizeof(Ctx) <= 128, "context ring");
+  auto ctx_at = [&](int it) -> Ctx* {
+    return reinterpret_cast<Ctx*>(smem + P::OFF_C + 128 * (it & 3));
+  };
   // Copies of tile `tile` into slot `slot`: the velocities (parts & 1), then q
   // (parts & 2) with q0 into L2, where the epilogue's loads find it (without:
   // stage 2 85.6 instead of 78.1 us at 32^3).
-  auto copy = [&](int tile, int slot, int parts) {
+  auto copy = [&](int it, int tile, int slot, int parts) {
     const Ctx t = context(tile);
+    if constexpr (BATCH) {
+      if (parts & 1) {
+        *ctx_at(it) = t;
+        if (tile + gridDim.x < ntiles) *ctx_at(it + 1) = context(tile + gridDim.x);
+      }
+    }
     const CUtensorMap* maps =
         BATCH ? static_cast<const CUtensorMap*>(A.insts[A.tiles[tile].inst].maps) : M.m;
     unsigned char* dst = smem + slot * P::SLOT;
@@ -222,7 +234,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     for (; lane == 0 && ahead < NS; ++ahead) {
       const int tile = blockIdx.x + ahead * gridDim.x;
       if (tile >= ntiles || tile + 1 == A.inject_skip) break;
-      copy(tile, ahead, 1);
+      copy(ahead, tile, ahead, 1);
     }
     pdl_wait();
     for (int it = 0; lane == 0; ++it) {
@@ -234,7 +246,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
         break;
       }
       if (tile + 1 == A.inject_skip) continue;  // test hook: leave the slot empty
-      copy(tile, slot, it < ahead ? 2 : 3);
+      copy(it, tile, slot, it < ahead ? 2 : 3);
     }
     return;
   }
@@ -318,6 +330,12 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     }
   };
 
+  // Context of the block's tile it (batched: once its copies are there).
+  auto of_tile = [&](int it, int tile) {
+    if constexpr (BATCH) return *ctx_at(it);
+    else return context(tile);
+  };
+
   float met = 0.0f;
   if (blockIdx.x < ntiles) {
     int row = 0;
@@ -332,8 +350,22 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     if (tile >= ntiles) break;
     const bool more = tile + gridDim.x < ntiles;
     const int slot = it % NS;
-    const Ctx C = context(tile);
-    const Ctx N = context(more ? tile + gridDim.x : tile);
+    if constexpr (BATCH) {  // the contexts come with the copies
+      const uint32_t parity = (it / NS) & 1;
+      const bool ok = mbar_wait_bounded(&full[slot], parity, A.wait_spins);
+      // The warps that share an element leave together, or none does.
+      if (!(H == 1 ? __all_sync(kAll, ok) != 0 : bar_and_warps(1 + es, 32 * H, ok))) {
+        // Wait for the copies still in flight (bounded) and leave.
+        if (lane == 0) {
+          atomicExch(A.status, kStatusWaitTimeout);
+          if (more) mbar_wait_bounded(&full[(it + 1) % NS], ((it + 1) / NS) & 1, A.wait_spins);
+          mbar_wait_bounded(&full[slot], parity, A.wait_spins);
+        }
+        return;
+      }
+    }
+    const Ctx C = of_tile(it, tile);
+    const Ctx N = more ? of_tile(it + 1, tile + gridDim.x) : C;
     const bool active = es < C.n;  // idle warps of a short tile keep pace
     const long base = static_cast<long>(C.e0 + (active ? es : 0)) * NP + (PAIR ? 2 * lane : 8 * zj + yi);
     unsigned char* st = smem + slot * P::SLOT;
@@ -352,17 +384,19 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
 #pragma unroll
     for (int f = 0; f < 6; ++f) hs[f] = 0.5f * __shfl_sync(kAll, met, 3 + f);
 
-    const uint32_t parity = (it / NS) & 1;
-    const bool ok = mbar_wait_bounded(&full[slot], parity, A.wait_spins);
-    // The warps that share an element leave together, or none does.
-    if (!(H == 1 ? __all_sync(kAll, ok) != 0 : bar_and_warps(1 + es, 32 * H, ok))) {
-      // Wait for the copies still in flight (bounded) and leave.
-      if (lane == 0) {
-        atomicExch(A.status, kStatusWaitTimeout);
-        if (more) mbar_wait_bounded(&full[(it + 1) % NS], ((it + 1) / NS) & 1, A.wait_spins);
-        mbar_wait_bounded(&full[slot], parity, A.wait_spins);
+    if constexpr (!BATCH) {
+      const uint32_t parity = (it / NS) & 1;
+      const bool ok = mbar_wait_bounded(&full[slot], parity, A.wait_spins);
+      // The warps that share an element leave together, or none does.
+      if (!(H == 1 ? __all_sync(kAll, ok) != 0 : bar_and_warps(1 + es, 32 * H, ok))) {
+        // Wait for the copies still in flight (bounded) and leave.
+        if (lane == 0) {
+          atomicExch(A.status, kStatusWaitTimeout);
+          if (more) mbar_wait_bounded(&full[(it + 1) % NS], ((it + 1) / NS) & 1, A.wait_spins);
+          mbar_wait_bounded(&full[slot], parity, A.wait_spins);
+        }
+        return;
       }
-      return;
     }
 
     // ---- Columns: q and the z-flux; w's place then takes the line sums -------
