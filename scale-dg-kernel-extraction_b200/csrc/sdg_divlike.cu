@@ -46,8 +46,17 @@
 namespace sdg {
 namespace {
 
+// Resident blocks the build must allow where that measured faster than the
+// compiler's own choice (0), us for 7.4 M values, gradient / five fields: p = 11
+// 61.5 / 65.8 with three blocks (66.8 / 72.0), p = 13 83 / 94 with two and the z
+// contraction first (109 / 112: 254 registers, one block of seven warps), p = 15
+// five fields 67.8 with two (72.5).  Elsewhere one to eight blocks measured no
+// better.
+template <int NQ, bool EXACT, bool ONE>
+constexpr int kDerivBlocks = EXACT ? 0 : NQ == 12 ? 3 : NQ == 14 ? 2 : (NQ == 16 && !ONE) ? 2 : 0;
+
 template <int NQ, bool EXACT, int ORDER, bool ONE>
-__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32)
+__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, kDerivBlocks<NQ, EXACT, ONE>)
     derivative_kernel(const double* __restrict__ ix, const double* __restrict__ iy,
                       const double* __restrict__ iz, double* __restrict__ ox,
                       double* __restrict__ oy, double* __restrict__ oz, long long units,
@@ -78,7 +87,8 @@ __global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32)
   // gradlike p = 8 149 / 126, p = 9 148 / 118; both operators p = 10-12
   // 109-146 / 93-133; five fields p = 7 125 / 144, p = 8 115 / 125, p = 9
   // 112 / 119; both p = 14 76-81 / 135-155.
-  constexpr bool EARLYZ = (NQ >= 11 && NQ <= 13) || (ONE && (NQ == 9 || NQ == 10));
+  constexpr bool EARLYZ = (NQ >= 11 && NQ <= 13) || (ONE && (NQ == 9 || NQ == 10)) ||
+                          (NQ == 14 && !EXACT);
   auto zderiv = [&](const double (&col)[NQ]) {
     // Z-dir (erb:430-463): vec_in_z(i,j,l) * Mat_tr(l,k), stored straight
     // from registers (coalesced over the warp).
