@@ -261,7 +261,10 @@ long long sdg_launch_count(sdg_handle* h);
  * (TMA) ring, 3 = one tile per block built for 8 resident blocks (p = 3..7),
  * 4 = the bulk-copy ring with each z-column split over two threads (p >= 8;
  * other orders run variant 2).  All compute identical results; the choice
- * only affects speed. */
+ * only affects speed.  At p = 7 the fast FP64 and mixed forms run their
+ * warp-per-element kernels whatever is asked for (but 5, the tensor-core
+ * experiment of the mixed form); at some orders the automatic variant is a
+ * kernel that cannot be asked for by number (the line kernel). */
 int sdg_set_kernel_variant(sdg_handle* h, int variant);
 
 /* Test hook for the failure path of the bounded waits (no reference
@@ -273,7 +276,7 @@ int sdg_set_kernel_variant(sdg_handle* h, int variant);
  * handle's status word and returns, and the next synchronising call
  * (sdg_synchronize, sdg_get_field, sdg_minmax) fails with SDG_ERR_CUDA and
  * clears the word.  tile < 0 restores normal operation; the handle stays
- * usable throughout.  Only the pipelined kernel variant has waits. */
+ * usable throughout.  The one-tile-per-block kernels have no waits. */
 int sdg_debug_inject_wait_timeout(sdg_handle* h, int tile, int spins);
 
 /* Host logic of sdg_rk3_steps_host and the chunked sdg_cal_tend, exposed
@@ -333,7 +336,8 @@ int sdg_batch_get(sdg_batch* b, int id, double* q);
 /* Up to n values: instances, total DOF, run seconds, DOF x steps run,
  * groups, then per group p, mixed, tiles, chosen variant and the tuned
  * stage times (ms) of the pipelined, block, 8-blocks-per-SM and
- * split-column variants (0 where not a candidate).
+ * split-column variants (0 where not a candidate; variant 6 is the line
+ * kernel, whose time is not listed).
  * Returns the number of values available. */
 int sdg_batch_info(sdg_batch* b, double* out, int n);
 

@@ -217,14 +217,14 @@ __device__ __forceinline__ float2 contract2(FA A, FB B) {
 // FP64 tensor-core line contractions (fast FP64 kernels, Nq = 8)
 // ---------------------------------------------------------------------------
 // The x- and y-derivatives of an element are the 8x8-by-8x64 products
-// D * F_x and D * F_y (over the 64 lines of each direction).  The fast FP64
-// kernels at Nq = 8 compute them with mma.sync m8n8k4 (DMMA): one 8x8 output
-// tile = one k-plane of the element, two chained k-steps (l = 0..3, then
-// 4..7).  A DMMA does 256 FMAs in one warp instruction where the DFMA form
+// D * F_x and D * F_y (over the 64 lines of each direction).  The
+// one-tile-per-block kernel, which the fast FP64 form at Nq = 8 runs where
+// Lift_mat does not factorise (else tend_warp_kernel), computes them with
+// mma.sync m8n8k4 (DMMA): one 8x8 output tile = one k-plane of the element, two
+// chained k-steps (l = 0..3, then 4..7).  A DMMA does 256 FMAs in one warp instruction where the DFMA form
 // needs 32 per instruction, at the same FP64 peak.  Fragments (PTX ISA,
 // m8n8k4 .f64): lane L holds A(L>>2, L&3), B(L&3, L>>2) and
-// C(L>>2, 2(L&3) + {0,1}).  Every kernel variant uses this same sequence,
-// so their fast FP64 results stay bit-identical.
+// C(L>>2, 2(L&3) + {0,1}).
 __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b,
                                             double c0, double c1) {
   asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%5};"

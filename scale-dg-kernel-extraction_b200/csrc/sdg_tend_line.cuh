@@ -230,10 +230,10 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
           copy(c.u, sizeof(TV) * NP, c, smem + P::OFF_U, fu, true);
           copy(c.v, sizeof(TV) * NP, c, smem + P::OFF_V, fv, true);
           copy(c.w, sizeof(TV) * NP, c, smem + P::OFF_W, fw, true);
-          pdl_wait();
         }
-        state(c, slot);
       }
+      if (it == 0) pdl_wait();
+      if (ok && !skip) state(c, slot);
       if (it > 0) {
         ok = ok && mbar_wait_bounded(eu, (it - 1) & 1, spins);
         if (ok && !skip) copy(c.u, sizeof(TV) * NP, c, smem + P::OFF_U, fu, true);
