@@ -167,6 +167,10 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
+# The stage kernel of the workloads at p = 7 (others: the pipelined kernel).
+STAGE_KERNEL = {"fp64_32c_p7": "tend_warp_kernel", "mixed_32c_p7": "tend_warp32_kernel"}
+
+
 def profiled_traffic(workload):
     """Per-launch DRAM bytes of the fused stage kernel from the committed ncu
     summary (profiles/<kernel>_<workload>.json), or None."""
@@ -347,7 +351,8 @@ def time_mesh(sdg, rep, name, steps, warmup, gidx):
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                         "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
                         "traffic": profiled_traffic(name),
-                        "kernel": "tend_pipe_kernel (fused flux+volume+lift+RK stage)",
+                        "kernel": STAGE_KERNEL.get(name, "tend_pipe_kernel") +
+                                  " (fused flux+volume+lift+RK stage)",
                         "stage_ms": stage_ms, "alg_bytes_per_dof": bpd},
            "clocks": clk.summary(), "gpu_launches": launches}
     return res, (H, ops, mesh, flags, fields, dt)
@@ -480,7 +485,7 @@ def time_batch(sdg, rep, mixed, steps, warmup, gidx, bf):
                        "l2": "inputs larger than L2 (no flush)"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
-                         "kernel": "tend_pipe_kernel, batched tile tables",
+                         "kernel": "tend_warp/line/pipe kernels, batched tile tables",
                          "alg_bytes_per_dof": bpd, "groups": groups},
             "clocks": clk.summary(),
             "gpu_launches": 3 * len(info["groups"]) * steps}
@@ -617,7 +622,7 @@ def time_served(sdg, rep, nreq, seq_sample, gidx):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
                          "over": "device-busy time",
-                         "kernel": "tend_pipe_kernel, batched tile tables"},
+                         "kernel": "tend_warp/line/pipe kernels, batched tile tables"},
             "clocks": clk.summary()}
 
 
