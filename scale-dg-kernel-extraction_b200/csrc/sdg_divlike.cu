@@ -34,7 +34,8 @@
 // (i,k) = (a,b) in place and its z-column in registers (at some orders the
 // z-column first, before the barrier), and after a second barrier it stores
 // its x and y output columns.  No scratch, no
-// atomics: every unit reads and writes only its own Np nodes.
+// atomics: every unit reads and writes only its own Np nodes.  At some orders
+// the y-lines go straight from and to global memory (derivative_half_kernel).
 #include <cuda_runtime.h>
 
 #include "sdg_gpu.h"
@@ -49,14 +50,13 @@ namespace {
 // Resident blocks the build must allow where that measured faster than the
 // compiler's own choice (0), us for 7.4 M values, gradient / five fields: p = 11
 // 61.5 / 65.8 with three blocks (66.8 / 72.0), p = 13 83 / 94 with two and the z
-// contraction first (109 / 112: 254 registers, one block of seven warps), p = 15
-// five fields 67.8 with two (72.5).  Elsewhere one to eight blocks measured no
-// better.
-template <int NQ, bool EXACT, bool ONE>
-constexpr int kDerivBlocks = EXACT ? 0 : NQ == 12 ? 3 : NQ == 14 ? 2 : (NQ == 16 && !ONE) ? 2 : 0;
+// contraction first (109 / 112: 254 registers, one block of seven warps).
+// Elsewhere one to eight blocks measured no better.
+template <int NQ, bool EXACT>
+constexpr int kDerivBlocks = EXACT ? 0 : NQ == 12 ? 3 : NQ == 14 ? 2 : 0;
 
 template <int NQ, bool EXACT, int ORDER, bool ONE>
-__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, kDerivBlocks<NQ, EXACT, ONE>)
+__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, kDerivBlocks<NQ, EXACT>)
     derivative_kernel(const double* __restrict__ ix, const double* __restrict__ iy,
                       const double* __restrict__ iz, double* __restrict__ ox,
                       double* __restrict__ oy, double* __restrict__ oz, long long units,
@@ -138,6 +138,80 @@ __global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, kDerivBlock
   }
 }
 
+// The y-lines straight from and to global memory: thread (a,b) of a unit is
+// y-line (i,k) = (a,b), whose loads and stores run over i in the warp (runs of Nq
+// words; the loads hit L1 where the unit's one input was just read), so only the
+// x-lines pass through shared memory: half the buffer, half the traffic there.
+// Same operations, same results.  The y input is read after z results are
+// written, so the caller keeps inputs and outputs apart (else the kernel above).
+// us for 7.4 M values, this kernel / the one above, gradient: p = 1 40.5 / 49.3, p = 2
+// 43.2 / 51.5, p = 4 41.6 / 44.3, p = 6 43.2 / 45.2, p = 7 39.1 / 44.5, p = 8 47.2 /
+// 49.3, p = 14 46.0 / 52.9, p = 15 42.9 / 55.7; five fields: p = 1 55.5 / 59.5, p = 2
+// 57.0 / 65.7, p = 4 56.0 / 61.6, p = 5 55.8 / 57.4, p = 14 59.0 / 63.5, p = 15 57.6 /
+// 72.5; equal or slower elsewhere (p = 9 52.4 / 51.2 and 80 / 65).  With the x-lines
+// straight from global memory as well: slower from p = 4 on (58.7, p = 9 57.6).
+template <int NQ, bool EXACT, bool ONE>
+constexpr bool kDerivHalf =
+    !EXACT && (NQ == 2 || NQ == 3 || NQ == 5 || NQ == 15 || NQ == 16 ||
+               (ONE ? NQ >= 7 && NQ <= 9 : NQ == 6));
+
+template <int NQ, int ORDER, bool ONE>
+__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, NQ == 15 ? 0 : 4)
+    derivative_half_kernel(const double* __restrict__ ix, const double* __restrict__ iy,
+                           const double* __restrict__ iz, double* __restrict__ ox,
+                           double* __restrict__ oy, double* __restrict__ oz, long long units,
+                           const __grid_constant__ DMat<NQ, double> D) {
+  using G = Geo<NQ>;
+  using LI = LineIdx<NQ, 8>;
+  using AR = Ar<double, false>;
+  constexpr int NQ2 = G::NQ2;
+  extern __shared__ __align__(16) double line_smem[];
+  const int s = threadIdx.x / NQ2;  // unit slot of the block
+  const int t = threadIdx.x - s * NQ2;
+  const int a = t % NQ;
+  const int b = t / NQ;
+  const long long u = static_cast<long long>(blockIdx.x) * G::EPB + s;
+  const bool active = s < G::EPB && u < units;
+  double* sX = line_smem + s * LI::SIZE;
+  const long long base = u * G::NP + t;
+  if (active) {
+    double col[NQ];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const double xv = ldro(ix + base + NQ2 * k);
+      sX[LI::colx(a, b, k)] = xv;
+      col[k] = ONE ? xv : ldro(iz + base + NQ2 * k);
+    }
+#pragma unroll
+    for (int k = 0; k < NQ; ++k)
+      oz[base + NQ2 * k] = contract<NQ, ORDER, AR, double>(
+          [&](int l) { return col[l]; }, [&](int l) { return D.d[k * NQ + l]; });
+  }
+  __syncthreads();
+  if (active) {
+    double line[NQ];
+    const int lbx = LI::xl_base(a, b);
+#pragma unroll
+    for (int l = 0; l < NQ; ++l) line[l] = sX[LI::xl(lbx, l)];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i)
+      sX[LI::xl(lbx, i)] = contract<NQ, ORDER, AR, double>(
+          [&](int l) { return D.d[i * NQ + l]; }, [&](int l) { return line[l]; });
+    const long long y0 = u * G::NP + a + NQ2 * b;
+#pragma unroll
+    for (int l = 0; l < NQ; ++l) line[l] = ldro(iy + y0 + NQ * l);
+#pragma unroll
+    for (int j = 0; j < NQ; ++j)
+      oy[y0 + NQ * j] = contract<NQ, ORDER, AR, double>(
+          [&](int l) { return line[l]; }, [&](int l) { return D.d[j * NQ + l]; });
+  }
+  __syncthreads();
+  if (active) {
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) ox[base + NQ2 * k] = sX[LI::colx(a, b, k)];
+  }
+}
+
 struct DerivCall {
   const double* ix;
   const double* iy;
@@ -150,11 +224,12 @@ struct DerivCall {
   cudaStream_t stream;
 };
 
-template <int NQ, bool EXACT, int ORDER, bool ONE>
-int launch_derivative(const DerivCall& c) {
+// Launches KERN over the units with `buffers` line buffers per unit.
+template <auto KERN, int NQ>
+int launch_units(const DerivCall& c, int buffers) {
   using G = Geo<NQ>;
-  auto kern = derivative_kernel<NQ, EXACT, ORDER, ONE>;
-  const size_t smem = sizeof(double) * 2 * LineIdx<NQ, 8>::SIZE * G::EPB;
+  constexpr auto kern = KERN;
+  const size_t smem = sizeof(double) * buffers * LineIdx<NQ, 8>::SIZE * G::EPB;
   static DeviceSetup setup;  // per instantiation and device
   const int dev = setup_device();
   if (dev < 0) return fail(SDG_ERR_CUDA, "derivative: no usable current device");
@@ -171,7 +246,7 @@ int launch_derivative(const DerivCall& c) {
   DMat<NQ, double> d;
   for (int i = 0; i < NQ; ++i)
     for (int l = 0; l < NQ; ++l) d.d[i * NQ + l] = c.D1D[i + NQ * l];  // D(i,l)
-  for (int i = 0; i < 2 * NQ; ++i) d.lz[i] = 0.0;
+  for (int i = 0; i < 2 * NQ; ++i) d.lz[i] = d.lx[i] = d.ly[i] = 0.0;
   const long long blocks = (c.units + G::EPB - 1) / G::EPB;
   if (blocks > 0x7fffffffLL) return fail(SDG_ERR_ARG, "derivative: too many elements");
   kern<<<static_cast<unsigned>(blocks), G::THREADS, smem, c.stream>>>(c.ix, c.iy, c.iz, c.ox,
@@ -180,6 +255,21 @@ int launch_derivative(const DerivCall& c) {
   if (e != cudaSuccess)
     return fail(SDG_ERR_CUDA, "derivative kernel launch failed: %s", cudaGetErrorString(e));
   return SDG_OK;
+}
+
+template <int NQ, bool EXACT, int ORDER, bool ONE>
+int launch_derivative(const DerivCall& c) {
+  if constexpr (kDerivHalf<NQ, EXACT, ONE>) {
+    // Outputs that share memory with an input take the other kernel.
+    const long long n = c.units * Geo<NQ>::NP;
+    const double* in[3] = {c.ix, c.iy, c.iz};
+    const double* out[3] = {c.ox, c.oy, c.oz};
+    bool apart = true;
+    for (const double* i : in)
+      for (const double* o : out) apart = apart && (o + n <= i || i + n <= o);
+    if (apart) return launch_units<derivative_half_kernel<NQ, ORDER, ONE>, NQ>(c, 1);
+  }
+  return launch_units<derivative_kernel<NQ, EXACT, ORDER, ONE>, NQ>(c, 2);
 }
 
 template <int NQ>
