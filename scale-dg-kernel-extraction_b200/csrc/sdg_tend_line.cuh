@@ -222,8 +222,11 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
         c.n = min(tw, A.nelem - tile * tw);
       }
       const int slot = it & 1;
-      bool ok = it < 2 || mbar_wait_bounded(done, it & 1, spins);
-      if (ok && !skip) {
+      // The slot is free: the iteration before waited for `done` of tile it - 2.
+      // (A second wait for that phase could find the barrier two phases on,
+      // where its parity reads as not yet complete.)
+      bool ok = true;
+      if (!skip) {
         rows(c, slot);
         if (it == 0) {
           // Velocities before the wait for the previous stage.
@@ -233,7 +236,7 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
         }
       }
       if (it == 0) pdl_wait();
-      if (ok && !skip) state(c, slot);
+      if (!skip) state(c, slot);
       if (it > 0) {
         ok = ok && mbar_wait_bounded(eu, (it - 1) & 1, spins);
         if (ok && !skip) copy(c.u, sizeof(TV) * NP, c, smem + P::OFF_U, fu, true);
