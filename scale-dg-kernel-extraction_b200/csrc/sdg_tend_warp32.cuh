@@ -85,6 +85,12 @@ __device__ __forceinline__ void tma_rows_g2s(void* dst, const CUtensorMap* map, 
       : "memory");
 }
 
+// Before a block's first use of a tensor map that the host copied to global
+// memory: what the copy wrote is what its tensor copies read.
+__device__ __forceinline__ void tensormap_acquire(const CUtensorMap* map) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.sys [%0], 128;" ::"l"(map) : "memory");
+}
+
 // Word index of node (i,j,k) in a swizzled element of floats or doubles.
 template <typename T>
 __device__ __forceinline__ int swz(int i, int j, int k) {
@@ -201,16 +207,23 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
   // Copies of tile `tile` into slot `slot`: the velocities (parts & 1), then q
   // (parts & 2) with q0 into L2, where the epilogue's loads find it (without:
   // stage 2 85.6 instead of 78.1 us at 32^3).
+  int acquired = -1;  // instance whose maps this block last acquired
   auto copy = [&](int it, int tile, int slot, int parts) {
     const Ctx t = context(tile);
+    const CUtensorMap* maps = M.m;
     if constexpr (BATCH) {
+      const int inst = A.tiles[tile].inst;
+      maps = static_cast<const CUtensorMap*>(A.insts[inst].maps);
       if (parts & 1) {
         *ctx_at(it) = t;
         if (tile + gridDim.x < ntiles) *ctx_at(it + 1) = context(tile + gridDim.x);
+        // The tables are rewritten in place when members come and go.
+        if (inst != acquired)
+#pragma unroll
+          for (int f = 0; f < 4; ++f) tensormap_acquire(maps + f);
+        acquired = inst;
       }
     }
-    const CUtensorMap* maps =
-        BATCH ? static_cast<const CUtensorMap*>(A.insts[A.tiles[tile].inst].maps) : M.m;
     unsigned char* dst = smem + slot * P::SLOT;
     constexpr int RQ = static_cast<int>(P::QB / 128), RV = static_cast<int>(P::VB / 128);
     if (parts & 1) {
