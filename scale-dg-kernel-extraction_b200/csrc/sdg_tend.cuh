@@ -289,6 +289,14 @@ template <typename T>
 __device__ __forceinline__ T ldro(const T* p) {
   return __ldg(p);
 }
+// A value of the state.  With programmatic dependent launch the stage before may
+// still be writing it when this kernel starts, so it is not constant over the
+// kernel as ldro's non-coherent loads require: a plain load, which stays behind
+// pdl_wait.
+template <typename T>
+__device__ __forceinline__ T ld_state(const T* p) {
+  return *p;
+}
 
 // ---------------------------------------------------------------------------
 // Kernel arguments
@@ -468,7 +476,7 @@ __global__ void __launch_bounds__(Geo<NQ>::THREADS, MINB)
       } else {
         idx = static_cast<long>(-1 - p) + t;
       }
-      const TC qP = static_cast<TC>(ldro(A.q + idx));
+      const TC qP = static_cast<TC>(ld_state(A.q + idx));
       const TC unP = static_cast<TC>((f == 1 || f == 3) ? ldro(A.u + idx)
                                                         : ldro(A.v + idx));
       const TC sg = (f == 0 || f == 3) ? TC(-1) : TC(1);
@@ -481,13 +489,13 @@ __global__ void __launch_bounds__(Geo<NQ>::THREADS, MINB)
       const int p5 = pb[4];
       const long i5 = (p5 >= 0) ? static_cast<long>(p5) + t + NQ2 * (NQ - 1)
                                 : static_cast<long>(-1 - p5) + t;
-      const TC q5 = static_cast<TC>(ldro(A.q + i5));
+      const TC q5 = static_cast<TC>(ld_state(A.q + i5));
       const TC w5 = static_cast<TC>(ldro(A.w + i5));
       f5 = upwind_flux<AR, TC>(qc[0], wlo, q5, w5, TC(-1), fs[4]);
       const int p6 = pb[5];
       const long i6 = (p6 >= 0) ? static_cast<long>(p6) + t
                                 : static_cast<long>(-1 - p6) + t;
-      const TC q6 = static_cast<TC>(ldro(A.q + i6));
+      const TC q6 = static_cast<TC>(ld_state(A.q + i6));
       const TC w6 = static_cast<TC>(ldro(A.w + i6));
       f6 = upwind_flux<AR, TC>(qc[NQ - 1], whi, q6, w6, TC(1), fs[5]);
     }

@@ -291,7 +291,7 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
       }
       const long idx = pb >= 0 ? static_cast<long>(pb) + opp_offset<NQ>(f, a, b)
                                : static_cast<long>(-1 - pb) + n;
-      qP[f] = static_cast<TC>(ldro(c.q + idx));
+      qP[f] = static_cast<TC>(ld_state(c.q + idx));
       vP[f] = static_cast<TC>((f == 1 || f == 3) ? ldro(c.u + idx)
                                                  : (f >= 4 ? ldro(c.w + idx) : ldro(c.v + idx)));
     }

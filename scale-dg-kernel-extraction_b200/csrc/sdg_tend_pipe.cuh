@@ -770,7 +770,7 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
         if (in_tile & (1u << f)) continue;
         const long idx = (pbc[f] >= 0) ? static_cast<long>(pbc[f]) + opp_offset<NQ>(f, a, b)
                                        : static_cast<long>(-1 - pbc[f]) + t;
-        qP[f] = static_cast<TC>(ldro(C.q + idx));
+        qP[f] = static_cast<TC>(ld_state(C.q + idx));
         unP[f] = static_cast<TC>((f == 1 || f == 3) ? ldro(C.u + idx) : ldro(C.v + idx));
       }
 #pragma unroll
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
         const int f = 4 + z;
         const long idx = (pbc[f] >= 0) ? static_cast<long>(pbc[f]) + opp_offset<NQ>(f, a, b)
                                        : static_cast<long>(-1 - pbc[f]) + t;
-        qZ[z] = static_cast<TC>(ldro(C.q + idx));
+        qZ[z] = static_cast<TC>(ld_state(C.q + idx));
         wZ[z] = static_cast<TC>(ldro(C.w + idx));
       }
     };

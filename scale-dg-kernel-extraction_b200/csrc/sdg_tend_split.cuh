@@ -402,7 +402,7 @@ __global__ void __launch_bounds__((SplitGeo<NQ, H>::THREADS + 31) / 32 * 32,
         const int sl = (f >= 4) ? 2 : ((f == 0 || f == 1) ? 0 : 1);
         const long idx = (pb >= 0) ? static_cast<long>(pb) + opp_offset<NQ>(f, a, b)
                                    : static_cast<long>(-1 - pb) + c;
-        qP[sl] = static_cast<TC>(ldro(C.q + idx));
+        qP[sl] = static_cast<TC>(ld_state(C.q + idx));
         unP[sl] = static_cast<TC>((f == 1 || f == 3) ? ldro(C.u + idx)
                                                      : ((f >= 4) ? ldro(C.w + idx)
                                                                  : ldro(C.v + idx)));

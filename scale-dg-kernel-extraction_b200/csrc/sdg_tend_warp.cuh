@@ -61,15 +61,25 @@ constexpr bool kWarpKernel = NQ == 8 && sizeof(TC) == 8 && !EXACT;
 
 // Loads that stay where they are written (asm volatile), so that the values
 // are on their way while the warp works; the compiler otherwise sinks them
-// towards their use.
+// towards their use.  The state is not constant over the kernel (ld_state).
 __device__ __forceinline__ double ld_early(const double* p) {
   double v;
   asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ double ld_early_state(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ double2 ld_early2(const double* p) {
   double2 v;
   asm volatile("ld.global.nc.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double2 ld_early_state2(const double* p) {
+  double2 v;
+  asm volatile("ld.global.v2.f64 {%0,%1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
   return v;
 }
 // q0 is read once, and in stage 3 it is the array the kernel writes.
@@ -265,7 +275,7 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     const double* pv = (yface ? t.v : t.u) + n0 + k0 * ks;
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
-      qP[k] = ld_early(pq + k * ks);
+      qP[k] = ld_early_state(pq + k * ks);
       vP[k] = ld_early(pv + k * ks);
     }
   };
@@ -278,10 +288,10 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
                                : static_cast<long>(-1 - pz)) + 2 * lane;
       // A halo face may start at an odd node.
       if (VEC && (n0 & 1) == 0) {
-        qZ[z] = ld_early2(t.q + n0);
+        qZ[z] = ld_early_state2(t.q + n0);
         wZ[z] = ld_early2(t.w + n0);
       } else {
-        qZ[z] = make_double2(ldro(t.q + n0), ldro(t.q + n0 + 1));
+        qZ[z] = make_double2(ld_state(t.q + n0), ld_state(t.q + n0 + 1));
         wZ[z] = make_double2(ldro(t.w + n0), ldro(t.w + n0 + 1));
       }
     }

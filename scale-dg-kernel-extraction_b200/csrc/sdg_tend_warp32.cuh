@@ -152,6 +152,11 @@ __device__ __forceinline__ float ld_early(const float* p) {
   asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
   return v;
 }
+__device__ __forceinline__ float ld_early_state(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
 
 template <typename TQ, typename TO, bool BATCH, int H>
 __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
@@ -285,10 +290,15 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
   // of the tile, else -1).
   V xq[2], xu[2], yq[2], yv[2], zq[2], zw[2];
   int in_x[2] = {-1, -1};
-  // Two values at p and p + d (one where the lane has one line).
-  auto early = [&](auto* p, int d) {
-    const float a = static_cast<float>(ld_early(p));
-    return L::make(a, PAIR ? static_cast<float>(ld_early(p + d)) : 0.0f);
+  // Two values at p and p + d (one where the lane has one line): of a velocity,
+  // of the state.
+  auto early = [&](const float* p, int d) {
+    const float a = ld_early(p);
+    return L::make(a, PAIR ? ld_early(p + d) : 0.0f);
+  };
+  auto early_state = [&](const TQ* p, int d) {
+    const float a = static_cast<float>(ld_early_state(p));
+    return L::make(a, PAIR ? static_cast<float>(ld_early_state(p + d)) : 0.0f);
   };
   auto gather = [&](const Ctx& t, int row) {
 #pragma unroll
@@ -300,7 +310,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       if (in_x[s] < 0) {
         const long n = p >= 0 ? static_cast<long>(p) + (s == 0 ? 7 : 0) + 8 * xj + 64 * xk
                               : static_cast<long>(-1 - p) + xj + 8 * xk;
-        xq[s] = early(t.q + n, p >= 0 ? 256 : 32);
+        xq[s] = early_state(t.q + n, p >= 0 ? 256 : 32);
         xu[s] = early(t.u + n, p >= 0 ? 256 : 32);
       }
     }
@@ -311,7 +321,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       const int p = __shfl_sync(kAll, row, s == 0 ? 0 : 2);
       const long n = p >= 0 ? static_cast<long>(p) + (s == 0 ? 56 : 0) + 64 * yk + yi
                             : static_cast<long>(-1 - p) + 8 * yk + yi;
-      yq[s] = early(t.q + n, 1);
+      yq[s] = early_state(t.q + n, 1);
       yv[s] = early(t.v + n, 1);
     }
 #pragma unroll
@@ -320,7 +330,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       const int p = __shfl_sync(kAll, row, 4 + s);
       const long n = (p >= 0 ? static_cast<long>(p) + (s == 0 ? 448 : 0)
                              : static_cast<long>(-1 - p)) + (PAIR ? 2 * lane : 8 * zj + yi);
-      zq[s] = early(t.q + n, 1);
+      zq[s] = early_state(t.q + n, 1);
       zw[s] = early(t.w + n, 1);
     }
   };
