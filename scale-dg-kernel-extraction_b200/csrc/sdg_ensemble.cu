@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "sdg_gpu.h"
+#include "sdg_grow.h"
 #include "sdg_internal.h"
 #include "sdg_launch.h"
 #include "sdg_tend.cuh"
@@ -415,22 +416,16 @@ struct Ensemble {
     }
     g->ntiles = static_cast<int>(g->h_tiles.size());
     const int b = g->cur ^ 1;  // the buffer no launch in flight reads
-    if (ni > g->inst_cap_buf[b]) {
-      if (g->d_insts_buf[b]) cudaFree(g->d_insts_buf[b]);
-      g->inst_cap_buf[b] = std::max(ni, 2 * g->inst_cap_buf[b]);
-      ENS_CUDA(cudaMalloc(&g->d_insts_buf[b], 3L * g->inst_cap_buf[b] * sizeof(BatchInst)));
-      if (g->warp && g->mixed) {
-        if (g->d_maps_buf[b]) cudaFree(g->d_maps_buf[b]);
-        g->d_maps_buf[b] = nullptr;
-        ENS_CUDA(cudaMalloc(&g->d_maps_buf[b], 3L * g->inst_cap_buf[b] * kFieldMapsBytes));
-      }
-    }
-    if (g->ntiles > g->tile_cap_buf[b]) {
-      if (g->d_tiles_buf[b]) cudaFree(g->d_tiles_buf[b]);
-      g->tile_cap_buf[b] = std::max(g->ntiles, 2 * g->tile_cap_buf[b]);
-      ENS_CUDA(cudaMalloc(&g->d_tiles_buf[b],
-                          static_cast<size_t>(g->tile_cap_buf[b]) * sizeof(BatchTile)));
-    }
+    auto alloc = [](void** p, size_t bytes) { return static_cast<int>(cudaMalloc(p, bytes)); };
+    const GrowTable insts[2] = {
+        {reinterpret_cast<void**>(&g->d_insts_buf[b]), 3 * sizeof(BatchInst)},
+        {reinterpret_cast<void**>(&g->d_maps_buf[b]), 3 * kFieldMapsBytes}};
+    const GrowTable tiles[1] = {
+        {reinterpret_cast<void**>(&g->d_tiles_buf[b]), sizeof(BatchTile)}};
+    ENS_CUDA(static_cast<cudaError_t>(grow_tables(ni, &g->inst_cap_buf[b], insts,
+                                                  g->warp && g->mixed ? 2 : 1, alloc, cudaFree)));
+    ENS_CUDA(static_cast<cudaError_t>(
+        grow_tables(g->ntiles, &g->tile_cap_buf[b], tiles, 1, alloc, cudaFree)));
     g->cur = b;
     g->d_insts = g->d_insts_buf[b];
     g->d_tiles = g->d_tiles_buf[b];
