@@ -236,18 +236,23 @@ int run(const LaunchSpec& s) {
     // blocks per SM: 216 elements 48 against 62 us a step, 512 112 against 122)
     // and in the exact forms (which wait for the lift table's loads one by one:
     // p = 11, 64 elements 25.4 against 27.1, 343 elements 61.5 against 53.9).
-    const bool few = (NQ == 16 || EXACT) && !batch && s.nelem > 0 &&
-                     s.nelem <= (EXACT ? 2 : 4) * (s.num_sms > 0 ? s.num_sms : 148);
-    if (can && !few && (s.variant == kVariantLine || (s.variant == kVariantAuto && !batch))) {
+    const int sms = s.num_sms > 0 ? s.num_sms : 148;
+    const bool few = (NQ == 16 || EXACT) && !batch && s.nelem <= (EXACT ? 2 : 4) * sms;
+    if (can && (s.variant == kVariantLine || (s.variant == kVariantAuto && !batch))) {
       // Shorter tiles where the longest would leave a block without one.
-      const int slots = LineTile<NQ, TC>::BLOCKS * (s.num_sms > 0 ? s.num_sms : 148);
+      const int slots = LineTile<NQ, TC>::BLOCKS * sms;
       a.tile_elems = std::max(1, std::min(LP::E, (s.nelem + slots - 1) / slots));
       const int ntiles = batch ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
       if (batch)
         return launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, true>,
                            LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);
-      return launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, false>,
-                         LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);
+      // (A call without elements primes this kernel and the one of few elements.)
+      if (!few || s.nelem <= 0) {
+        const int rc =
+            launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, false>,
+                        LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);
+        if (rc != 0 || !few) return rc;
+      }
     }
   }
   // The split-column kernel: orders with one element per tile.
