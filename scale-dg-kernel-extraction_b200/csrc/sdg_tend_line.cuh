@@ -226,17 +226,21 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
       // (A second wait for that phase could find the barrier two phases on,
       // where its parity reads as not yet complete.)
       bool ok = true;
+      // Velocities before the wait for the previous stage.
+      const bool q_last = it == 0 && A.chained;
       if (!skip) {
         rows(c, slot);
+        if (!q_last) state(c, slot);
         if (it == 0) {
-          // Velocities before the wait for the previous stage.
           copy(c.u, sizeof(TV) * NP, c, smem + P::OFF_U, fu, true);
           copy(c.v, sizeof(TV) * NP, c, smem + P::OFF_V, fv, true);
           copy(c.w, sizeof(TV) * NP, c, smem + P::OFF_W, fw, true);
         }
       }
-      if (it == 0) pdl_wait();
-      if (!skip) state(c, slot);
+      if (q_last) {
+        pdl_wait();
+        if (!skip) state(c, slot);
+      }
       if (it > 0) {
         ok = ok && mbar_wait_bounded(eu, (it - 1) & 1, spins);
         if (ok && !skip) copy(c.u, sizeof(TV) * NP, c, smem + P::OFF_U, fu, true);
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
     }
   };
 
-  pdl_wait();
+  if (A.chained) pdl_wait();
   if (blockIdx.x < ntiles) {
     if (!mbar_wait_bounded(&fq[0], 0, spins)) atomicExch(A.status, kStatusWaitTimeout);
     else gather(0);

@@ -504,7 +504,7 @@ constexpr int pipe_min_blocks() {
 // line owner reads its eight results back into the line buffers.  Its
 // rounding differs from the FP32 FMA lines of the other variants.
 template <int NQ, typename TQ, typename TV, typename TO, typename TC, bool EXACT,
-          int ORDER, bool STAGE, bool BATCH, bool TCG = false>
+          int ORDER, bool STAGE, bool BATCH, bool TCG = false, bool PDL = false>
 __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
                                   (pipe_min_blocks<NQ, TQ, TV, TC, EXACT, STAGE, TCG, BATCH>()))
     tend_pipe_kernel(const __grid_constant__ TendArgs<TQ, TV, TO, TC> A,
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
   static_assert(!(NQ == 8 && sizeof(TC) == 8 && !EXACT),
                 "fast FP64 at Nq = 8: tend_warp_kernel");
 
-  if constexpr (kPdl<NQ>) pdl_trigger();
+  if constexpr (PDL) pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char* slots = smem_raw;
   TC* sL = reinterpret_cast<TC*>(smem_raw + NS * P::SLOT + P::FACE);
@@ -589,29 +589,19 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
       tile_range(c.e0, c.n, sizeof(int) * 6, &plo, &pby, &psh);
       total += pby;
     }
-    if constexpr (!kPdl<NQ>) {
-      mbar_arrive_expect_tx(&bars[slot], total);
+    if (parts & 1) mbar_arrive_expect_tx(&bars[slot], total);
+    if (parts & 2)
+      bulk_g2s(base, static_cast<const unsigned char*>(src[0]) + lo[0], by[0], &bars[slot]);
+    if (parts & 1) {
 #pragma unroll
-      for (int k = 0; k < 6; ++k)
+      for (int k = 1; k < 6; ++k)
         bulk_g2s(base + off[k], static_cast<const unsigned char*>(src[k]) + lo[k], by[k],
                  &bars[slot]);
       if constexpr (RCTX)
         bulk_g2s(base + P::OFF_P, reinterpret_cast<const unsigned char*>(c.pbase) + plo, pby,
                  &bars[slot]);
-    } else {
-      if (parts & 1) {
-        mbar_arrive_expect_tx(&bars[slot], total);
-#pragma unroll
-        for (int k = 1; k < 6; ++k)
-          bulk_g2s(base + off[k], static_cast<const unsigned char*>(src[k]) + lo[k], by[k],
-                   &bars[slot]);
-        if constexpr (RCTX)
-          bulk_g2s(base + P::OFF_P, reinterpret_cast<const unsigned char*>(c.pbase) + plo, pby,
-                   &bars[slot]);
-      }
-      if (!(parts & 2)) return;
-      bulk_g2s(base, static_cast<const unsigned char*>(src[0]) + lo[0], by[0], &bars[slot]);
     }
+    if (!(parts & 2)) return;
     // q0 (RK stages 2-3) is read by the epilogue straight from global
     // memory; bring the tile's range into L2 now.
     if (STAGE && A.rk_a != 0.0) {
@@ -655,17 +645,20 @@ __global__ void __launch_bounds__((PipeGeo<NQ>::THREADS + 31) / 32 * 32,
     tc::fence_after_sync();
     tmem = *tmem_slot;
   }
-  if (kPdl<NQ> && threadIdx.x == 0)
-    for (int k = 0; k < NS; ++k) {
-      const int tile = blockIdx.x + k * gridDim.x;
-      if (tile < ntiles) issue(tile, k, 1);
+  // Chained: what no stage writes, the wait for the previous stage, then q; else
+  // all at once.
+  const bool chained = PDL && A.chained;
+  if (threadIdx.x == 0) {
+    for (int pass = chained ? 0 : 1; pass < 2; ++pass) {
+      if (pass == 1 && chained) pdl_wait();
+      for (int k = 0; k < NS; ++k) {
+        const int tile = blockIdx.x + k * gridDim.x;
+        if (tile < ntiles) issue(tile, k, pass == 0 ? 1 : (chained ? 2 : 3));
+      }
     }
-  if constexpr (kPdl<NQ>) pdl_wait();
-  if (threadIdx.x == 0)
-    for (int k = 0; k < NS; ++k) {
-      const int tile = blockIdx.x + k * gridDim.x;
-      if (tile < ntiles) issue(tile, k, kPdl<NQ> ? 2 : 3);
-    }
+  } else if (chained) {
+    pdl_wait();
+  }
 
   for (int it = 0;; ++it) {
     const int tile = blockIdx.x + it * gridDim.x;

@@ -212,12 +212,12 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     // warps are done with tile it - NS.
     // The first tiles' velocities go before the wait for the previous stage.
     int ahead = 0;
-    for (; VEC && lane == 0 && ahead < NS; ++ahead) {
+    for (; VEC && A.chained && lane == 0 && ahead < NS; ++ahead) {
       const int tile = blockIdx.x + ahead * gridDim.x;
       if (tile >= ntiles || tile + 1 == A.inject_skip) break;
       copy(ahead, 1);
     }
-    pdl_wait();
+    if (A.chained) pdl_wait();
     for (int it = 0; VEC && lane == 0; ++it) {
       const int tile = blockIdx.x + it * gridDim.x;
       if (tile >= ntiles) break;
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     int row = 0;
     const Ctx t = context(blockIdx.x);
     load_row(t, &row, &met);
-    pdl_wait();
+    if (A.chained) pdl_wait();
     gather(t, row);
     gather_z(t, row);
   }

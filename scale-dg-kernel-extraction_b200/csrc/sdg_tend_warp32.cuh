@@ -249,12 +249,12 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
   if (warp == P::WARPS) {
     // Producer, as in tend_warp_kernel.
     int ahead = 0;
-    for (; lane == 0 && ahead < NS; ++ahead) {
+    for (; A.chained && lane == 0 && ahead < NS; ++ahead) {
       const int tile = blockIdx.x + ahead * gridDim.x;
       if (tile >= ntiles || tile + 1 == A.inject_skip) break;
       copy(ahead, tile, ahead, 1);
     }
-    pdl_wait();
+    if (A.chained) pdl_wait();
     for (int it = 0; lane == 0; ++it) {
       const int tile = blockIdx.x + it * gridDim.x;
       if (tile >= ntiles) break;
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     int row = 0;
     const Ctx t = context(blockIdx.x);
     load_row(t, &row, &met);
-    pdl_wait();
+    if (A.chained) pdl_wait();
     gather(t, row);
   }
 
