@@ -233,12 +233,11 @@ int run(const LaunchSpec& s) {
                      (batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) && aligned(s.w) &&
                                 aligned(s.escale) && aligned(s.fscale) && aligned(s.pbase) &&
                                 (s.q0 == nullptr || aligned(s.q0))));
-    // Small meshes stay with the kernels before it at Nq = 16 (which run two
-    // blocks per SM: 216 elements 48 against 62 us a step, 512 112 against 122)
-    // and in the exact forms (which wait for the lift table's loads one by one:
-    // p = 11, 64 elements 25.4 against 27.1, 343 elements 61.5 against 53.9).
     const int sms = s.num_sms > 0 ? s.num_sms : 148;
-    const bool few = (NQ == 16 || EXACT) && !batch && s.nelem <= (EXACT ? 2 : 4) * sms;
+    const bool prime = s.nelem <= 0 && !batch;
+    const bool few = !batch && (prime ? kLineFew<NQ, EXACT>
+                                      : line_few<NQ, TC, EXACT, STAGE>(s.nelem, sms, s.pdl,
+                                                                       s.nelem < s.Ne));
     if (can && (s.variant == kVariantLine || (s.variant == kVariantAuto && !batch))) {
       // Shorter tiles where the longest would leave a block without one.
       const int slots = LineTile<NQ, TC>::BLOCKS * sms;
@@ -247,8 +246,9 @@ int run(const LaunchSpec& s) {
       if (batch)
         return launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, true>,
                            LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);
-      // (A call without elements primes this kernel and the one of few elements.)
-      if (!few || s.nelem <= 0) {
+      // (A call without elements primes this kernel and the one
+      // that launches of few elements take.)
+      if (!few || prime) {
         const int rc =
             launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, false>,
                         LP::THREADS>(LP::BYTES, ntiles, s, a, d, 0, true);

@@ -64,6 +64,48 @@ template <int NQ, typename TC, bool EXACT>
 constexpr bool kLineAuto =
     EXACT ? NQ >= 12 && NQ <= 14 : NQ == 2 || (sizeof(TC) == 8 && NQ >= 10);
 
+// Whether a launch of n elements of one instance stays with the kernels before
+// this one (`part`: some of a mesh's elements; `chained`: a programmatic dependent
+// launch, whose barrier set-up and first copies hide behind the stage before).
+// us per launch at 148 SMs, this kernel / the one before, on boxes near a cube:
+//   p = 1        tiles of a few elements, four threads each, with their own set-up
+//                and seven copies.  FP64 chained 1728 elements 2.75 / 2.60, 2548 2.76
+//                / 2.77, 4096 2.83 / 3.51; single stages 4624 3.61 / 3.23, 5000 3.69
+//                / 3.91; tendency 4624 3.39 / 3.08, 5508 3.44 / 3.74.  Mixed chained
+//                4096 2.84 / 2.40, 4624 2.82 / 2.79, 5508 2.83 / 3.42; single stages
+//                9240 3.76 / 3.47, 10000 3.88 / 3.93.
+//   p = 9, 11, 12  single stages, whose first tile nothing hides: p = 9 64 elements
+//                5.22 / 5.02, 294 6.45 / 6.28, 343 and more faster; p = 11 64 6.08 /
+//                5.94, p = 12 80 7.29 / 6.75, 140 and more equal or faster.  Chained
+//                ones are faster from the start (p = 9 64 4.78 / 5.05).  A part of a
+//                host-buffer call follows another part's launch that it does not
+//                read: five steps of 9^3 at p = 9 443 / 481 us.
+//   p = 10       single stages and parts 64 6.33 / 5.43, 252 equal; chained 64 equal,
+//                80 5.94 / 5.41, 144 7.03 / 5.64 (blocks of the next stage share the
+//                SM), 180 to 294 equal, 343 7.83 / 10.09.  And where the second round
+//                of three blocks an SM is a third full while that of two is full: 576
+//                13.16 / 12.27; 448 10.84 / 11.88, 648 13.49 / 14.96.
+//   p = 15       one block an SM against two: 64 10.77 / 10.54, 216 19.76 / 15.45, 512
+//                40.05 / 36.82, 592 equal.
+//   exact        the lift table's loads one by one: p = 11 64 7.60 / 7.29 (single 8.25 /
+//                7.29), 144 7.69 / 7.85; p = 12 single 64 9.48 / 9.20.
+template <int NQ, typename TC, bool EXACT, bool STAGE>
+inline bool line_few(long n, long sms, bool chained, bool part) {
+  constexpr bool F64 = sizeof(TC) == 8;
+  const bool single = STAGE && !chained && !part;
+  long per = 0;  // elements per SM
+  if (EXACT) per = 2;
+  else if (NQ == 16) per = 4;
+  else if (NQ == 2) per = chained ? (F64 ? 17 : 30) : F64 ? 32 : 64;
+  else if (NQ == 11) per = STAGE ? 2 : 0;
+  else if (NQ == 10) per = single ? 2 : 0;
+  else if (NQ == 12 || NQ == 13) per = single ? 1 : 0;
+  return n <= per * sms || (NQ == 11 && !EXACT && STAGE && 2 * n > 7 * sms && n <= 4 * sms);
+}
+// The orders and forms at which it may.
+template <int NQ, bool EXACT>
+constexpr bool kLineFew = EXACT || NQ == 2 || (NQ >= 10 && NQ <= 13) || NQ == 16;
+
 template <int NQ, typename TQ, typename TV, typename TC>
 struct LinePlan {
   using LT = LineTile<NQ, TC>;
