@@ -3,46 +3,50 @@
 //
 // A k-plane of an element is an 8x8 (j, i) block.  Lane L = 4g + c of the warp
 // holds nodes (i = 2c, 2c+1; j = g) of each of the eight planes: 16-byte
-// words, consecutive over the lanes, which is at once the C-fragment layout of
-// mma.sync m8n8k4 (rows j, columns i) and, with the contraction index taken as
-// l = 2c + s in step s, the A fragment of an x-line product.  So
+// words, consecutive over the lanes, which is the C-fragment layout of mma.sync
+// m8n8k4 (rows j, columns i).  So
 //
-//   x   C(j,i) += sum_l Fx(l,j) D(i,l)   A = Fx from registers, B = D
-//   y   C(j,i) += sum_l D(j,l) Fy(i,l)   A = D, B = Fy, whose fragments the
-//                                        warp transposes through shared memory
-//   x/y lift   C(j,i) += l1(j) f1(i) + l3(j) f3(i) + f4(j) l4(i) + f2(j) l2(i)
-//                                        one k-step: A = (l1,l3,f4,f2)(j),
-//                                        B = (f1,f3,l4,l2)(i)
+//   x   C(j,i) = sum_l Fx(l,j) D(i,l)   A = Fx, formed from q and u at l = c and
+//                                       c + 4 of row g, B = D
+//   y   C(j,i) = sum_l D(j,l) Fy(i,l)   A = D, B = Fy, whose fragments the warp
+//                                       transposes through shared memory
+//   x/y lift   C(j,i) = l1(j) f1(i) + f2(j) l2(i) + l3(j) f3(i) + f4(j) l4(i)
+//                                       one k-step: A = (l1,f2,l3,f4)(j),
+//                                       B = (f1,l2,f3,l4)(i)
 //   z   each lane holds whole columns: eight FMAs per node from registers,
 //       and the two z-lift terms
 //
-// accumulate in the same registers, and the RK update and the store follow
-// from there.  In the lift step lane (g, c) needs exactly one face flux per
-// plane, that of face node (g, k) of face c in (-y, +y, -x, +x), and computes
-// it itself: no flux goes through shared memory, and no phase needs more than
-// one warp, so there is no block barrier.  The metric factors (and, in RK
-// stages, dt and the stage coefficient) are folded into D, w and the flux
-// scale, once per element.
+// meet in the lane that updates and stores the node.  In the lift step lane (g, c)
+// needs exactly one face flux per plane, that of face node (g, k) of face c in
+// (-y, +x, +y, -x), and computes it itself: no flux goes through shared memory, and
+// no phase needs more than one warp, so there is no block barrier.
+//
+// The tensor core adds its four products one after another in ascending l, each
+// with one rounding (checked against FMA chains), so every node's operations and
+// their order are those of tend_kernel, and so are the bits.  (With l = 2c + s in
+// step s the A fragments of x come from registers, and with dt, the stage
+// coefficient and the metric factors folded into D, w and the flux scale the sums
+// need no scaling: meshes of 1,000 to 8,000 elements took 3 to 10 % less, 32^3 the
+// same, but each folded operand is a rounding more: 2.37e-16 instead of 2.13e-16
+// against 64 bits after five steps.)
 //
 // A tile is up to seven consecutive elements, one per warp; an eighth warp
 // keeps a ring of two tiles (q, u, v, w: 16 KB an element) filled by bulk
 // copies, full/empty mbarriers between it and the seven, one block per SM.  A
-// slot is refilled, two tiles ahead, once every warp holds its q and its sums.
+// slot is refilled, two tiles ahead, once every warp has its sums.
 // The Fy transposition reuses the element's own w, which is in registers by
 // then; q, u and v stay as copied, so a face neighbour in the same tile is
 // read from shared memory.  The other plus-side values come from global memory
 // (L2), loaded a tile ahead.  Every bounded wait and the status word work as
 // in tend_pipe_kernel.
 //
-// Measured (32^3 elements, us per launch of RK stage 1 / 2 / 3): 120 / 130 /
-// 129 against 153 / 160 / 160 for the block kernel it replaced (two warps per
-// element, line buffers and fluxes in shared memory), i.e. 5.6 / 6.2 / 6.2 TB/s
-// of the 40 / 48 / 48 algorithmic bytes per node, where a copy reaches 6.5.
-// Shared-memory pipe 75 -> 37 % busy; seven warps per SM, about 980
-// instructions per element.  Tried on the way: seven independent warps with a
-// ring each and all face values from L2, 153 / 183 / 183 (the -x/+x faces are
-// 8-byte words 64 bytes apart, each a 32-byte sector); without any
-// neighbour's values 111 / 130.
+// Measured (32^3 elements): 123 / 134 / 133 us per single launch of RK stage 1 / 2 /
+// 3 and 375 us a chained step, against 153 / 160 / 160 and 469 for the block kernel
+// it replaced (two warps per element, line buffers and fluxes in shared memory); the
+// step is 6.1 TB/s of the 40 / 48 / 48 algorithmic bytes per node, where a copy
+// reaches 6.56.  Tried on the way: seven independent warps with a ring each and all
+// face values from L2, 153 / 183 / 183 (the -x/+x faces are 8-byte words 64 bytes
+// apart, each a 32-byte sector); without any neighbour's values 111 / 130.
 //
 // H warps per element (1, 2 or 4): the latency form for meshes too small to
 // give every warp of the GPU an element.  Warp h of an element takes planes
@@ -124,9 +128,6 @@ __device__ __forceinline__ bool bar_and_warps(int id, int threads, bool ok) {
   return r != 0;
 }
 
-// Arithmetic of an element: -dqdt's sign, dt and rk_b are folded into the
-// scale `sc`, so acc is the increment of rk_b * q (RK stages) or dqdt itself.
-//
 // VEC: the arrays are 16-byte aligned (bulk copies and 16-byte accesses);
 // otherwise the warp fills its slot with plain loads and stores word by word.
 template <bool STAGE, bool BATCH, bool VEC, int H>
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
   constexpr size_t EB = NP * sizeof(double);  // bytes of an element's field
   constexpr int NS = VEC ? P::NSTAGE : 1;
   constexpr unsigned kAll = 0xffffffffu;
+  using AR = Ar<double, false>;
   pdl_trigger();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + P::NSTAGE * P::SLOT + P::EXCH);
@@ -232,22 +234,23 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     return;
   }
 
-  // Face of this lane: c = 0, 1, 2, 3: -y, +y, -x, +x (0-based faces 0, 2, 3,
-  // 1), face node (g, k); minus- and plus-side node of plane k = 0.
-  const int face = c == 0 ? 0 : (c == 1 ? 2 : (c == 2 ? 3 : 1));
-  const int moff = c == 0 ? g : (c == 1 ? g + 56 : (c == 2 ? 8 * g : 8 * g + 7));
-  const int poff = c == 0 ? g + 56 : (c == 1 ? g : (c == 2 ? 8 * g + 7 : 8 * g));
-  const bool yface = c < 2;
-  const double sgn = (c == 0 || c == 2) ? -1.0 : 1.0;
+  // Face of this lane: c = 0, 1, 2, 3: -y, +x, +y, -x, the order of the lift's
+  // sum, face node (g, k); minus- and plus-side node of plane k = 0.
+  const int face = c;
+  const int moff = c == 0 ? g : (c == 1 ? 8 * g + 7 : (c == 2 ? g + 56 : 8 * g));
+  const int poff = c == 0 ? g + 56 : (c == 1 ? 8 * g : (c == 2 ? g : 8 * g + 7));
+  const bool yface = (c & 1) == 0;
+  const double sgn = (c == 0 || c == 3) ? -1.0 : 1.0;
   // Lift factor l_f of this lane's face at normal index g (faces -y, +y along
   // j; -x, +x along i).
   const double lf = ldro(A.lift + NP * face + ((face & 1) ? g : 8 * g));
-  // D fragments: x: D(i = g, l = 2c + s); y: D(j = g, l = c + 4s).
-  double dx[2], dy[2];
-  dx[0] = D.d[8 * g + 2 * c];
-  dx[1] = D.d[8 * g + 2 * c + 1];
-  dy[0] = D.d[8 * g + c];
-  dy[1] = D.d[8 * g + c + 4];
+  // D fragments: D(g, c) and D(g, c + 4), B of the x and A of the y products.
+  const double d0 = D.d[8 * g + c], d1 = D.d[8 * g + c + 4];
+  // x fragments: nodes i = c, c + 4 of row j = g.  The lanes of every other pair
+  // of rows read them in the other order, which keeps the loads free of bank
+  // conflicts.
+  const bool swap = (g & 2) != 0;
+  const int xa = 8 * g + (swap ? c + 4 : c), xb = 8 * g + (swap ? c : c + 4);
 
   // Face-neighbour row (lanes 0-5) and metric factors (lanes 0-2 escale, 3-8
   // fscale) of a tile, one word per lane, shared out by shuffles: loaded a
@@ -296,12 +299,12 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
       }
     }
   };
-  // Scaled upwind flux: sg (qP vP - qM vM) - |vP + vM| / 2 (qP - qM), times
-  // fscale / 2 (mod_advect3d_eq.f90:134-139).
-  auto flux = [](double qM, double vM, double qp, double vp, double c1, double c2) {
-    const double u = fma(qp, vp, -__dmul_rn(qM, vM));
-    const double h = __dmul_rn(fabs(__dadd_rn(vp, vM)), __dsub_rn(qp, qM));
-    return fma(c2, h, __dmul_rn(c1, u));
+  // upwind_flux (sdg_tend.cuh), rounded alike: the sign factors out of the
+  // products exactly; hs = fscale / 2.
+  auto flux = [](double qM, double vM, double qp, double vp, double sg, double hs) {
+    const double t = AR::sub(AR::mul(qp, vp), AR::mul(qM, vM));
+    const double alpha = AR::mul(0.5, fabs(AR::add(vp, vM)));
+    return AR::mul(hs, fma(sg, t, -AR::mul(alpha, AR::sub(qp, qM))));
   };
 
   // Waits for the slot of the block's tile it (bounded); false: leave.
@@ -374,17 +377,12 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
     double met_n = 0.0;
     load_row(N, &row_n, &met_n);
 
-    // Metric factors and, folded into them, the sign and the RK weight.
-    const double sc = STAGE ? -(C.dt * A.rk_b) : -1.0;
-    const double scaled = met * sc;
-    const double E1 = __shfl_sync(kAll, scaled, 0);
-    const double E2 = __shfl_sync(kAll, scaled, 1);
-    const double E3 = __shfl_sync(kAll, scaled, 2);
-    const double fsf = __shfl_sync(kAll, scaled, 3 + face);
-    const double fsz0 = __shfl_sync(kAll, scaled, 7);
-    const double fsz1 = __shfl_sync(kAll, scaled, 8);
-    const double bx0 = dx[0] * E1, bx1 = dx[1] * E1;
-    const double ay0 = dy[0] * E2, ay1 = dy[1] * E2;
+    const double e1 = __shfl_sync(kAll, met, 0);
+    const double e2 = __shfl_sync(kAll, met, 1);
+    const double e3 = __shfl_sync(kAll, met, 2);
+    const double hsf = AR::mul(0.5, __shfl_sync(kAll, met, 3 + face));
+    const double hsz0 = AR::mul(0.5, __shfl_sync(kAll, met, 7));
+    const double hsz1 = AR::mul(0.5, __shfl_sync(kAll, met, 8));
 
     // ---- The element's q, u, v, w ------------------------------------------
     if constexpr (VEC) {
@@ -402,10 +400,10 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
       __syncwarp();
     }
 
-    // acc: this warp's planes; fz: the whole columns.
-    double acc[2 * KP], fz[16], q[2 * KP];
+    // q: this warp's planes; fz: the whole columns of q*w.
+    double fz[16], q[2 * KP];
     double ql[2], qh[2], wl[2], wh[2];
-    // ---- Volume fluxes, x products, Fy to its transposition buffer ---------
+    // ---- Fluxes of the z columns, Fy to its transposition buffer ------------
     constexpr int KG = KP < 4 ? KP : 4;
 #pragma unroll
     for (int h = 0; h < KP / KG; ++h) {
@@ -414,26 +412,21 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
       for (int kk = 0; kk < KG; ++kk) {
         const int k = KG * h + kk, n = 64 * (k0 + k) + 2 * lane;
         const double2 q2 = *reinterpret_cast<const double2*>(sq + n);
-        const double2 u2 = *reinterpret_cast<const double2*>(su + n);
         const double2 v2 = *reinterpret_cast<const double2*>(sv + n);
         const double2 w2 = *reinterpret_cast<const double2*>(sw + n);
         q[2 * k] = q2.x;
         q[2 * k + 1] = q2.y;
         if (H == 1 && k == 0) { wl[0] = w2.x; wl[1] = w2.y; }
         if (H == 1 && k == 7) { wh[0] = w2.x; wh[1] = w2.y; }
-        const double z0 = __dmul_rn(__dmul_rn(q2.x, w2.x), E3);
-        const double z1 = __dmul_rn(__dmul_rn(q2.y, w2.y), E3);
+        const double z0 = AR::mul(q2.x, w2.x), z1 = AR::mul(q2.y, w2.y);
         if constexpr (H == 1) {
           fz[2 * k] = z0;
           fz[2 * k + 1] = z1;
         } else {
           *reinterpret_cast<double2*>(sz + n) = make_double2(z0, z1);
         }
-        fy[2 * kk] = __dmul_rn(q2.x, v2.x);
-        fy[2 * kk + 1] = __dmul_rn(q2.y, v2.y);
-        double c0, c1;
-        dmma_m8n8k4(c0, c1, __dmul_rn(q2.x, u2.x), bx0, 0.0, 0.0);
-        dmma_m8n8k4(acc[2 * k], acc[2 * k + 1], __dmul_rn(q2.y, u2.y), bx1, c0, c1);
+        fy[2 * kk] = AR::mul(q2.x, v2.x);
+        fy[2 * kk + 1] = AR::mul(q2.y, v2.y);
       }
       __syncwarp();  // every lane has read its w of these planes
       // F_y(i,j) of plane k at 64k + 8j + 2((i>>1) ^ (j&2)) + (i&1): the pair
@@ -465,7 +458,23 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
       }
     }
 
-    // ---- y products, face fluxes and the x/y lift ---------------------------
+    // ---- z-derivative and z fluxes -------------------------------------------
+    // D(k,l) and the z-lift factors: constant-bank operands where the plane is
+    // known at compile time (H = 1), uniform loads otherwise.
+    double dz[2 * KP];
+#pragma unroll
+    for (int k = 0; k < 2 * KP; ++k) {
+      dz[k] = AR::mul(fz[k & 1], D.d[8 * (k0 + (k >> 1))]);
+#pragma unroll
+      for (int l = 1; l < 8; ++l)
+        dz[k] = AR::mad(fz[2 * l + (k & 1)], D.d[8 * (k0 + (k >> 1)) + l], dz[k]);
+    }
+    const double f5[2] = {flux(ql[0], wl[0], qZ[0].x, wZ[0].x, -1.0, hsz0),
+                          flux(ql[1], wl[1], qZ[0].y, wZ[0].y, -1.0, hsz0)};
+    const double f6[2] = {flux(qh[0], wh[0], qZ[1].x, wZ[1].x, 1.0, hsz1),
+                          flux(qh[1], wh[1], qZ[1].y, wZ[1].y, 1.0, hsz1)};
+
+    // ---- x and y products, lift, RK update and store, plane by plane ---------
     const double* sf = yface ? sv : su;
     if (inside >= 0) {
       const double* nq = tq + inside + poff + 64 * k0;
@@ -476,67 +485,58 @@ __global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
         vP[k] = nf[64 * k];
       }
     }
-    const double cf1 = 0.5 * fsf * sgn, cf2 = -0.25 * fsf;
     const int yb = 8 * c + 2 * ((g >> 1) ^ (c & 2)) + (g & 1);
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
       const int n = 64 * (k0 + k);
-      const double b0 = sy[n + yb], b1 = sy[n + yb + 32];
-      const double f = flux(sq[n + moff], sf[n + moff], qP[k], vP[k], cf1, cf2);
-      double c0, c1;
-      dmma_m8n8k4(c0, c1, ay0, b0, acc[2 * k], acc[2 * k + 1]);
-      dmma_m8n8k4(c0, c1, ay1, b1, c0, c1);
-      dmma_m8n8k4(acc[2 * k], acc[2 * k + 1], yface ? lf : f, yface ? f : lf, c0, c1);
+      const double ga = AR::mul(sq[n + xa], su[n + xa]), gb = AR::mul(sq[n + xb], su[n + xb]);
+      double x0, x1, y0, y1, l0, l1;
+      dmma_m8n8k4(x0, x1, swap ? gb : ga, d0, 0.0, 0.0);
+      dmma_m8n8k4(x0, x1, swap ? ga : gb, d1, x0, x1);
+      dmma_tile8(d0, d1, sy[n + yb], sy[n + yb + 32], &y0, &y1);
+      const double f = flux(sq[n + moff], sf[n + moff], qP[k], vP[k], sgn, hsf);
+      dmma_m8n8k4(l0, l1, yface ? lf : f, yface ? f : lf, 0.0, 0.0);
+      const double xs[2] = {x0, x1}, ys[2] = {y0, y1}, ls[2] = {l0, l1};
+      // The results take dz's place: no branch parts the planes here.
+#pragma unroll
+      for (int m = 0; m < 2; ++m) {
+        const double lt = AR::mad(D.lz[8 + k0 + k], f6[m], AR::mad(D.lz[k0 + k], f5[m], ls[m]));
+        double acc = AR::mad(e2, ys[m], AR::mul(e1, xs[m]));
+        acc = AR::mad(e3, dz[2 * k + m], acc);
+        double r = -AR::add(acc, lt);
+        // q = rk_a*q0 + rk_b*(q + dt*dqdt), main.f90:70-71.
+        if constexpr (STAGE) r = AR::mul(A.rk_b, AR::mad(C.dt, r, q[2 * k + m]));
+        dz[2 * k + m] = r;
+      }
     }
-    const double cl1 = -0.5 * fsz0, ch1 = 0.5 * fsz1, cl2 = -0.25 * fsz0, ch2 = -0.25 * fsz1;
-    const double f5[2] = {flux(ql[0], wl[0], qZ[0].x, wZ[0].x, cl1, cl2),
-                          flux(ql[1], wl[1], qZ[0].y, wZ[0].y, cl1, cl2)};
-    const double f6[2] = {flux(qh[0], wh[0], qZ[1].x, wZ[1].x, ch1, ch2),
-                          flux(qh[1], wh[1], qZ[1].y, wZ[1].y, ch1, ch2)};
     // This warp is done with the slot: the next copies may overwrite it.
     fence_proxy_async_smem();
     __syncwarp();
     if (VEC && lane == 0) mbar_arrive(&empty[slot]);
-    // The next element's plus-side values, used an iteration on.
+    // The next element's plus-side values: on their way through the first half
+    // of the next iteration.
     if (more) {
       gather(N, row_n);
       gather_z(N, row_n);
     }
     met = met_n;
 
-    // ---- z-derivative, z lift, RK update, store ------------------------------
-    // D(k,l) and the z-lift factors: constant-bank operands where the plane is
-    // known at compile time (H = 1), uniform loads otherwise.
+    if (use_q0) {
 #pragma unroll
-    for (int k = 0; k < 2 * KP; ++k) {
-      acc[k] = fma(D.lz[k0 + (k >> 1)], f5[k & 1], acc[k]);
-      acc[k] = fma(D.lz[8 + k0 + (k >> 1)], f6[k & 1], acc[k]);
+      for (int k = 0; k < KP; ++k) {
+        dz[2 * k] = AR::mad(A.rk_a, q0[k].x, dz[2 * k]);
+        dz[2 * k + 1] = AR::mad(A.rk_a, q0[k].y, dz[2 * k + 1]);
+      }
     }
-#pragma unroll
-    for (int l = 0; l < 8; ++l)
-#pragma unroll
-      for (int k = 0; k < 2 * KP; ++k)
-        acc[k] = fma(D.d[8 * (k0 + (k >> 1)) + l], fz[2 * l + (k & 1)], acc[k]);
+    if (!active) continue;
 #pragma unroll
     for (int k = 0; k < KP; ++k) {
-      double r[2];
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        double s = acc[2 * k + m];
-        if constexpr (STAGE) {
-          // q = rk_a*q0 + rk_b*(q + dt*dqdt), main.f90:70-71.
-          s = fma(A.rk_b, q[2 * k + m], s);
-          if (use_q0) s = fma(A.rk_a, m == 0 ? q0[k].x : q0[k].y, s);
-        }
-        r[m] = s;
-      }
-      if (!active) continue;
       double* o = C.out + base + 64 * k;
       if constexpr (VEC) {
-        *reinterpret_cast<double2*>(o) = make_double2(r[0], r[1]);
+        *reinterpret_cast<double2*>(o) = make_double2(dz[2 * k], dz[2 * k + 1]);
       } else {
-        o[0] = r[0];
-        o[1] = r[1];
+        o[0] = dz[2 * k];
+        o[1] = dz[2 * k + 1];
       }
     }
   }
