@@ -260,11 +260,12 @@ long long sdg_launch_count(sdg_handle* h);
  * 1 = one element tile per block, 2 = persistent blocks with a bulk-copy
  * (TMA) ring, 3 = one tile per block built for 8 resident blocks (p = 3..7),
  * 4 = the bulk-copy ring with each z-column split over two threads (p >= 8;
- * other orders run variant 2).  All compute identical results; the choice
- * only affects speed.  At p = 7 the fast FP64 and mixed forms run their
- * warp-per-element kernels whatever is asked for (but 5, the tensor-core
- * experiment of the mixed form); at some orders the automatic variant is a
- * kernel that cannot be asked for by number (the line kernel). */
+ * other orders run variant 2), 5 = the tensor-core lines of the mixed form at
+ * p = 7 (an experiment with other rounding; elsewhere the automatic variant).
+ * The others compute identical results; the choice only affects speed.  At some
+ * orders the automatic variant is a kernel that cannot be asked for by number:
+ * the line kernel, and at p = 7 the warp-per-element kernels of the fast FP64
+ * and mixed forms (in FP64 also what 2 and 4 run). */
 int sdg_set_kernel_variant(sdg_handle* h, int variant);
 
 /* Test hook for the failure path of the bounded waits (no reference

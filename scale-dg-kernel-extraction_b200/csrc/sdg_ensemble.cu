@@ -559,8 +559,8 @@ struct Ensemble {
   // The kernel variants a group's launches support.
   std::vector<int> candidates(const Group* g) const {
     std::vector<int> cands;
-    // One kernel whatever the variant: launched as the pipelined one.
-    if (g->warp) return {kVariantPipe};
+    // The warp-per-element kernel is launched as the pipelined one.
+    if (g->warp) return {kVariantPipe, kVariantBlock, kVariantBlockOcc};
     if (g->line) cands.push_back(kVariantLine);
     const bool can_pipe = pipe_supported(g->nq, g->mixed ? kStageMixed2 : kStageF64) &&
                           pipe_supported(g->nq, g->mixed ? kStageMixed1 : kStageF64) &&
@@ -603,7 +603,8 @@ struct Ensemble {
       if (g->members.empty()) continue;
       int rc = rebuild(g);
       if (rc) return rc;
-      const std::vector<int> cands = candidates(g);
+      std::vector<int> cands = candidates(g);
+      if (g->warp) cands.resize(1);  // faster than the block kernels at every size
       cudaEvent_t e0, e1;
       ENS_CUDA(cudaEventCreate(&e0));
       ENS_CUDA(cudaEventCreate(&e1));

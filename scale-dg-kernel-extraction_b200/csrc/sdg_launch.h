@@ -106,9 +106,8 @@ int batch_elems_per_tile(int nq, bool mixed, bool exact, bool factored, int vari
 // Whether the line kernel (sdg_tend_line.cuh) is built for this order and form.
 bool line_kernel(int nq, bool mixed, bool exact, bool factored);
 
-// Whether the fast FP64 or mixed form of this order runs a warp-per-element
-// kernel (sdg_tend_warp.cuh, sdg_tend_warp32.cuh), whatever variant is asked
-// for.
+// Whether the fast FP64 or mixed form of this order has a warp-per-element
+// kernel (sdg_tend_warp.cuh, sdg_tend_warp32.cuh).
 bool warp_kernel(int nq, bool mixed, bool exact, bool factored);
 // Elements per tile: FP64, mixed.
 constexpr int kWarpElems = 7;
@@ -134,10 +133,12 @@ int launch_tend(const LaunchSpec& s);
 
 // Kernel variants: the one-tile-per-block kernel (tend_kernel) and the
 // persistent bulk-copy pipelined kernel (tend_pipe_kernel); identical
-// arithmetic.  Auto picks the split-column kernel at the orders where it
-// measured faster (kSplitAuto), else the pipelined one when its
-// shared-memory plan fits one block (kPipeMaxSmem) and every array is
-// 16-byte aligned, else the one-tile-per-block kernel.
+// arithmetic.  Auto picks the warp-per-element kernels at Nq = 8 (fast FP64 and
+// mixed), the line kernel where it measured faster (kLineAuto, line_few), the
+// split-column kernel likewise (kSplitAuto), else the pipelined one when its
+// shared-memory plan fits one block (kPipeMaxSmem) and every array is 16-byte
+// aligned, else the one-tile-per-block kernel.  The fast FP64 form at Nq = 8 has
+// no pipelined kernel but tend_warp_kernel.
 // kVariantBlockOcc is the one-tile-per-block kernel built for eight resident
 // blocks per SM (p = 3..7; other orders use kVariantBlock).
 // kVariantSplit is the persistent ring kernel with each z-column split over

@@ -176,11 +176,11 @@ __device__ __forceinline__ T contract(FA A, FB B) {
 // Orders (NQ = p + 1) whose fast FP32 kernels advance the x and y lines of a
 // thread together with packed FMAs (contract2).  Measured per order on the
 // pipelined kernel (G DOF-updates/s, paired vs scalar): p = 3 104.2 / 102.5,
-// p = 10 128.5 / 121.2, p = 11 111.4 / 102.3, p = 12
+// p = 7 146.7 / 140.7, p = 10 128.5 / 121.2, p = 11 111.4 / 102.3, p = 12
 // 119.9 / 99.4; slower at p = 4, 5, 8 (101.5 / 106.0, 106.7 / 114.1,
 // 109.1 / 118.7), where the wider live range costs a resident block.
 template <int NQ>
-constexpr bool kPairedLinesPipe = NQ == 4 || NQ >= 11;
+constexpr bool kPairedLinesPipe = NQ == 4 || NQ == 8 || NQ >= 11;
 // The one-tile-per-block kernel, which the fast FP32 forms run at p >= 13:
 // p = 13 78.2 / 63.5, p = 14 81.9 / 78.1, p = 15 92.7 / 86.9.
 template <int NQ>
@@ -219,12 +219,13 @@ __device__ __forceinline__ float2 contract2(FA A, FB B) {
 // FP64 tensor-core line contractions (fast FP64 kernels, Nq = 8)
 // ---------------------------------------------------------------------------
 // The x- and y-derivatives of an element are the 8x8-by-8x64 products
-// D * F_x and D * F_y (over the 64 lines of each direction).  The
-// one-tile-per-block kernel, which the fast FP64 form at Nq = 8 runs where
-// Lift_mat does not factorise (else tend_warp_kernel), computes them with
-// mma.sync m8n8k4 (DMMA): one 8x8 output tile = one k-plane of the element, two
-// chained k-steps (l = 0..3, then 4..7).  A DMMA does 256 FMAs in one warp instruction where the DFMA form
-// needs 32 per instruction, at the same FP64 peak.  Fragments (PTX ISA,
+// D * F_x and D * F_y (over the 64 lines of each direction).  The fast FP64
+// kernels at Nq = 8 (tend_warp_kernel; the one-tile-per-block kernel where it is
+// asked for or Lift_mat does not factorise) compute them with mma.sync m8n8k4
+// (DMMA): one 8x8 output tile = one k-plane of the element, two chained k-steps
+// (l = 0..3, then 4..7).  A DMMA does 256 FMAs in one warp instruction where the
+// DFMA form needs 32 per instruction, at the same FP64 peak.  Both use this same
+// sequence, so their results are bit-identical.  Fragments (PTX ISA,
 // m8n8k4 .f64): lane L holds A(L>>2, L&3), B(L&3, L>>2) and
 // C(L>>2, 2(L&3) + {0,1}).
 __device__ __forceinline__ void dmma_m8n8k4(double& d0, double& d1, double a, double b,

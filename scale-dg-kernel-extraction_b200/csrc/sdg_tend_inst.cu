@@ -176,10 +176,12 @@ int run(const LaunchSpec& s) {
                         (EXACT || s.lift_z != nullptr) &&
                         (batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) &&
                                    aligned(s.w) && aligned(s.escale) && aligned(s.fscale)));
-  // Fast FP64 at Nq = 8 with a factored lift: one warp per element, for
-  // every requested variant (bulk copies where the arrays are aligned).
+  // The one-tile-per-block kernels, asked for.
+  const bool block = !batch && (s.variant == kVariantBlock || s.variant == kVariantBlockOcc);
+  // Fast FP64 at Nq = 8 with a factored lift: one warp per element (bulk copies
+  // where the arrays are aligned), which is also this form's pipelined kernel.
   if constexpr (WARP) {
-    if (s.lift_z != nullptr && WarpPlan<1>::BYTES <= device_smem_optin()) {
+    if (s.lift_z != nullptr && !block && WarpPlan<1>::BYTES <= device_smem_optin()) {
       const bool vec = batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) && aligned(s.w) &&
                                  aligned(s.out) && (s.q0 == nullptr || aligned(s.q0)));
       const int sms = s.num_sms > 0 ? s.num_sms : 148;
@@ -204,10 +206,11 @@ int run(const LaunchSpec& s) {
       return launch_warp<tend_warp_kernel<STAGE, false, true, 1>, 1>(tiles(7), s, a, d);
     }
   }
-  // The mixed form at Nq = 8, likewise (but for the tensor-core experiment).
+  // The mixed form at Nq = 8, likewise, where no other kernel is asked for.
   if constexpr (STAGE && kWarp32Kernel<NQ, TC, EXACT>) {
-    if (s.lift_z != nullptr && (batch || s.field_maps != nullptr) &&
-        s.variant != kVariantTensor && Warp32Plan<TQ, 1>::BYTES <= device_smem_optin()) {
+    if (s.lift_z != nullptr &&
+        (batch || (s.field_maps != nullptr && s.variant == kVariantAuto)) &&
+        Warp32Plan<TQ, 1>::BYTES <= device_smem_optin()) {
       FieldMaps m;
       std::memset(&m, 0, sizeof(m));
       if (batch) return launch_warp32<tend_warp32_kernel<TQ, TO, true, 1>, TQ, 1>(s, a, d, m);
@@ -299,14 +302,16 @@ int run(const LaunchSpec& s) {
   const bool pipe =
       batch || ((s.variant == kVariantPipe || s.variant == kVariantAuto ||
                  s.variant == kVariantSplit || s.variant == kVariantTensor) && can_pipe);
-  if constexpr (!WARP && !(STAGE && kWarp32Kernel<NQ, TC, EXACT>)) if (pipe) {
+  if constexpr (!WARP) if (pipe) {
     const int ntiles =
         batch ? s.batch_ntiles : (s.nelem + PipeGeo<NQ>::EPB - 1) / PipeGeo<NQ>::EPB;
     constexpr bool PDL = STAGE && kPdl<NQ>;
-    if (batch)
-      return launch_pipe<
-          tend_pipe_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, true, false, PDL>>(
-          PB::BYTES, ntiles, s, a, d, 0, PDL);
+    if constexpr (!(STAGE && kWarp32Kernel<NQ, TC, EXACT>)) {
+      if (batch)
+        return launch_pipe<
+            tend_pipe_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, true, false, PDL>>(
+            PB::BYTES, ntiles, s, a, d, 0, PDL);
+    }
     // Chained launches have a kernel of their own: what they add costs the others
     // 2-4 % (mixed p = 5, 256,000 nodes 4.60 -> 4.80 us).  (A call without
     // elements primes both.)
