@@ -74,24 +74,28 @@ int launch_pipe(size_t smem, int ntiles, const LaunchSpec& s, const Args& a, con
   return launch_kernel(kern, grid, THREADS, smem, s, pdl, a, d);
 }
 
-// Launches the warp-per-element kernel: one block per SM, or one per tile
-// where there are fewer.
-template <auto KERN, int H, typename Args, typename Dm>
-int launch_warp(int ntiles, const LaunchSpec& s, const Args& a, const Dm& d) {
-  constexpr auto kern = KERN;
+// Launches the warp-per-element kernel with H warps an element and tiles of E
+// elements, or fewer where that leaves an SM without one: one block per SM, or
+// one per tile where there are fewer.
+template <bool STAGE, bool BATCH, bool VEC, int H, int E, typename Args, typename Dm>
+int launch_warp(const LaunchSpec& s, Args& a, const Dm& d) {
+  constexpr auto kern = tend_warp_kernel<STAGE, BATCH, VEC, H, E>;
+  using P = WarpPlan<H, E>;
   static DeviceSetup setup;  // per kernel and device
   const int dev = setup_device();
   if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
   if (setup.slot[dev].load(std::memory_order_relaxed) == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(WarpPlan<H>::BYTES));
+                                         static_cast<int>(P::BYTES));
     if (e != cudaSuccess) return static_cast<int>(e);
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     setup.slot[dev].store(1, std::memory_order_relaxed);
   }
+  const int sms = s.num_sms > 0 ? s.num_sms : 148;
+  a.tile_elems = std::max(1, std::min(E, (s.nelem + sms - 1) / sms));
+  const int ntiles = BATCH ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
   if (ntiles <= 0) return 0;
-  const int grid = std::min(ntiles, s.num_sms > 0 ? s.num_sms : 148);
-  return launch_kernel(kern, grid, WarpPlan<H>::THREADS, WarpPlan<H>::BYTES, s, true, a, d);
+  return launch_kernel(kern, std::min(ntiles, sms), P::THREADS, P::BYTES, s, true, a, d);
 }
 
 // The mixed form's warp-per-element kernel: tiles of the most elements a slot
@@ -118,13 +122,34 @@ int launch_warp32(const LaunchSpec& s, Args& a, const Dm& d, const FieldMaps& m)
   return launch_kernel(kern, std::min(ntiles, sms), P::THREADS, P::BYTES, s, true, a, d, m);
 }
 
-// Warps per element of the warp-per-element kernel for a mesh of `per_sm`
-// elements per SM: the split forms while one round of tiles holds them (one
-// element a tile with four warps, three with two).  Measured, us per RK step
-// from the step graph with H = 1 / 2 / 4: 64 elements 18.8 / 16.6 / 12.5, 148
-// 20.7 / 16.6 / 14.5, 296 20.7 / 16.6 / 18.6, 444 20.7 / 18.6 / 22.7, 592 20.7
-// / 24.8 / 26.8, 1036 20.7 / 30.9 / 37.1.
-inline int warps_per_elem(int per_sm) { return per_sm <= 1 ? 4 : (per_sm <= 3 ? 2 : 1); }
+// Warps per element of the warp-per-element kernel and elements per tile for a
+// mesh of `per_sm` elements per SM: the split forms while one round of their tiles
+// holds it, and two rounds of four elements where a round of seven would be
+// followed by one of one.  us per single stage / per chained one, with (warps,
+// elements) = (4,1) 64 elements 3.96 / 2.63; (4,2) 64 4.41 / 3.19, 252 4.64 / 3.53;
+// (2,3) 252 5.11 / 3.86, 392 5.10 / 3.95; (2,4) 392 5.59 / 4.47, 576 5.62 / 4.62, 1100
+// 8.64 / 7.29; (1,7) 576 6.38 / 5.23, 729 6.47 / 5.36, 1100 10.14 / 8.25.  (Nine
+// warps leave a thread 168 registers instead of 255.)
+enum class WarpForm { k41, k42, k23, k24, k17 };
+inline WarpForm warp_form(int per_sm) {
+  return per_sm <= 1   ? WarpForm::k41
+         : per_sm == 2 ? WarpForm::k42
+         : per_sm == 3 ? WarpForm::k23
+         : per_sm == 4 || per_sm == 8 ? WarpForm::k24
+                                      : WarpForm::k17;
+}
+
+// Mixed form at Nq = 8: whether a launch of n elements that is not chained stays
+// with the pipelined kernel: its 64 threads an element have a shorter way from the
+// first copy to the store than one or two warps, and its rounds of two elements a
+// block fill the SMs better where a round of eleven is followed by a short one.  us
+// per single stage, warp / pipelined: 64 elements 4.42 / 3.60, 576 4.61 / 4.37, 729
+// 4.78 / 4.98, 810 5.87 / 4.96, 1100 5.95 / 5.91, 1452 6.60 / 7.22, 1872 10.04 / 8.17,
+// 2548 10.31 / 9.88, 4096 13.85 / 14.32.
+inline bool warp32_few(long n, long sms, bool chained) {
+  return !chained && n > 0 &&
+         (n <= 4 * sms || (n > 5 * sms && 2 * n <= 15 * sms) || (n > 11 * sms && n <= 18 * sms));
+}
 
 template <typename TQ, typename TV, typename TO, typename TC, bool EXACT,
           int ORDER, bool STAGE>
@@ -181,35 +206,31 @@ int run(const LaunchSpec& s) {
   // Fast FP64 at Nq = 8 with a factored lift: one warp per element (bulk copies
   // where the arrays are aligned), which is also this form's pipelined kernel.
   if constexpr (WARP) {
-    if (s.lift_z != nullptr && !block && WarpPlan<1>::BYTES <= device_smem_optin()) {
+    if (s.lift_z != nullptr && !block && WarpPlan<1, kWarpElems>::BYTES <= device_smem_optin()) {
       const bool vec = batch || (aligned(s.q) && aligned(s.u) && aligned(s.v) && aligned(s.w) &&
                                  aligned(s.out) && (s.q0 == nullptr || aligned(s.q0)));
+      if (batch) return launch_warp<STAGE, true, true, 1, kWarpElems>(s, a, d);
+      if (!vec) return launch_warp<STAGE, false, false, 1, kWarpElems>(s, a, d);
       const int sms = s.num_sms > 0 ? s.num_sms : 148;
-      const int per_sm = (s.nelem + sms - 1) / sms;
-      // Tiles of the most elements the warps take, or fewer where that leaves
-      // an SM without one.
-      auto tiles = [&](int most) {
-        a.tile_elems = std::max(1, std::min(most, per_sm));
-        return batch ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
-      };
-      if (!vec && !batch)
-        return launch_warp<tend_warp_kernel<STAGE, false, false, 1>, 1>(tiles(7), s, a, d);
-      if (batch) return launch_warp<tend_warp_kernel<STAGE, true, true, 1>, 1>(tiles(7), s, a, d);
-      // (A call without elements primes every form.)
-      const int h = warps_per_elem(per_sm);
+      const WarpForm form = warp_form((s.nelem + sms - 1) / sms);
+      const bool prime = s.nelem <= 0;  // a call without elements primes every form
       int rc = 0;
-      if (h == 4 || s.nelem <= 0)
-        rc = launch_warp<tend_warp_kernel<STAGE, false, true, 4>, 4>(tiles(1), s, a, d);
-      if (rc == 0 && (h == 2 || s.nelem <= 0))
-        rc = launch_warp<tend_warp_kernel<STAGE, false, true, 2>, 2>(tiles(3), s, a, d);
-      if (rc != 0 || (h != 1 && s.nelem > 0)) return rc;
-      return launch_warp<tend_warp_kernel<STAGE, false, true, 1>, 1>(tiles(7), s, a, d);
+      auto take = [&](WarpForm f, auto launch) {
+        if (rc == 0 && (prime || form == f)) rc = launch();
+      };
+      take(WarpForm::k41, [&] { return launch_warp<STAGE, false, true, 4, 1>(s, a, d); });
+      take(WarpForm::k42, [&] { return launch_warp<STAGE, false, true, 4, 2>(s, a, d); });
+      take(WarpForm::k23, [&] { return launch_warp<STAGE, false, true, 2, 3>(s, a, d); });
+      take(WarpForm::k24, [&] { return launch_warp<STAGE, false, true, 2, 4>(s, a, d); });
+      take(WarpForm::k17, [&] { return launch_warp<STAGE, false, true, 1, kWarpElems>(s, a, d); });
+      return rc;
     }
   }
   // The mixed form at Nq = 8, likewise, where no other kernel is asked for.
   if constexpr (STAGE && kWarp32Kernel<NQ, TC, EXACT>) {
     if (s.lift_z != nullptr &&
-        (batch || (s.field_maps != nullptr && s.variant == kVariantAuto)) &&
+        (batch || (s.field_maps != nullptr && s.variant == kVariantAuto &&
+                   !warp32_few(s.nelem, s.num_sms > 0 ? s.num_sms : 148, s.pdl))) &&
         Warp32Plan<TQ, 1>::BYTES <= device_smem_optin()) {
       FieldMaps m;
       std::memset(&m, 0, sizeof(m));
@@ -218,14 +239,15 @@ int run(const LaunchSpec& s) {
       // Two warps an element while one round of tiles of five holds the mesh:
       // us per RK step with one / two warps, 64 elements 18.7 / 14.6, 740 18.6
       // / 14.6, 888 18.6 / 20.7, 1628 20.7 / 28.9.  (A call without elements
-      // primes both forms.)
+      // primes both forms and the kernel of warp32_few.)
       const int sms = s.num_sms > 0 ? s.num_sms : 148;
       const bool split = s.nelem <= sms * Warp32Plan<TQ, 2>::ELEMS;
-      if (split) {
-        const int rc = launch_warp32<tend_warp32_kernel<TQ, TO, false, 2>, TQ, 2>(s, a, d, m);
-        if (rc != 0 || s.nelem > 0) return rc;
-      }
-      return launch_warp32<tend_warp32_kernel<TQ, TO, false, 1>, TQ, 1>(s, a, d, m);
+      int rc = 0;
+      if (split || s.nelem <= 0)
+        rc = launch_warp32<tend_warp32_kernel<TQ, TO, false, 2>, TQ, 2>(s, a, d, m);
+      if (rc == 0 && (!split || s.nelem <= 0))
+        rc = launch_warp32<tend_warp32_kernel<TQ, TO, false, 1>, TQ, 1>(s, a, d, m);
+      if (rc != 0 || s.nelem > 0) return rc;
     }
   }
   // The line kernel.
@@ -397,7 +419,7 @@ int pipe_fits() {
     if (sb <= kPipeMaxSmem && sb <= optin) r |= 2;
   }
   if constexpr (kWarpKernel<NQ, TC, false>) {
-    if (WarpPlan<1>::BYTES <= optin) r |= 4;
+    if (WarpPlan<1, kWarpElems>::BYTES <= optin) r |= 4;
   }
   if constexpr (STAGE && kWarp32Kernel<NQ, TC, false>) {
     if (Warp32Plan<TQ, 1>::BYTES <= optin) r |= 4;

@@ -93,11 +93,11 @@ __device__ __forceinline__ double2 ld_early_stream2(const double* p) {
   return v;
 }
 
-template <int H>
+template <int H, int E>
 struct WarpPlan {
   static constexpr int NQ = 8;
   static constexpr int NP = 512;
-  static constexpr int ELEMS = kWarpElems / H;  // per tile at most
+  static constexpr int ELEMS = E;               // per tile at most
   static constexpr int WARPS = ELEMS * H;       // consumer warps
   static constexpr int NSTAGE = 2;
   static constexpr int THREADS = 32 * (WARPS + 1);
@@ -108,7 +108,8 @@ struct WarpPlan {
   static constexpr size_t OFF_C = NSTAGE * SLOT + EXCH + 16 * NSTAGE;
   static constexpr size_t BYTES = OFF_C + 4 * 128;  // four batched tiles' contexts
 };
-static_assert(WarpPlan<1>::BYTES <= kPipeMaxSmem, "warp kernel: shared memory");
+static_assert(WarpPlan<1, kWarpElems>::BYTES <= kPipeMaxSmem &&
+                  WarpPlan<2, 4>::BYTES <= kPipeMaxSmem, "warp kernel: shared memory");
 
 // Barriers of the `threads` threads of some warps: a plain one, and one that
 // also gives each of them whether all came with `ok`.
@@ -130,11 +131,11 @@ __device__ __forceinline__ bool bar_and_warps(int id, int threads, bool ok) {
 
 // VEC: the arrays are 16-byte aligned (bulk copies and 16-byte accesses);
 // otherwise the warp fills its slot with plain loads and stores word by word.
-template <bool STAGE, bool BATCH, bool VEC, int H>
-__global__ void __launch_bounds__(WarpPlan<H>::THREADS, 1)
+template <bool STAGE, bool BATCH, bool VEC, int H, int E>
+__global__ void __launch_bounds__((WarpPlan<H, E>::THREADS), 1)
     tend_warp_kernel(const __grid_constant__ TendArgs<double, double, double, double> A,
                      const __grid_constant__ DMat<8, double> D) {
-  using P = WarpPlan<H>;
+  using P = WarpPlan<H, E>;
   static_assert(H == 1 || VEC, "plain loads: one warp per element");
   constexpr int KP = 8 / H;   // planes of a warp
   using Ctx = TileCtx<double, double, double, double>;
