@@ -139,16 +139,18 @@ inline WarpForm warp_form(int per_sm) {
                                       : WarpForm::k17;
 }
 
-// Mixed form at Nq = 8: whether a launch of n elements that is not chained stays
-// with the pipelined kernel: its 64 threads an element have a shorter way from the
-// first copy to the store than one or two warps, and its rounds of two elements a
-// block fill the SMs better where a round of eleven is followed by a short one.  us
-// per single stage, warp / pipelined: 64 elements 4.42 / 3.60, 576 4.61 / 4.37, 729
-// 4.78 / 4.98, 810 5.87 / 4.96, 1100 5.95 / 5.91, 1452 6.60 / 7.22, 1872 10.04 / 8.17,
-// 2548 10.31 / 9.88, 4096 13.85 / 14.32.
+// Mixed form at Nq = 8: whether a launch of n elements stays with the pipelined
+// kernel: its 64 threads an element have a shorter way from the first copy to the
+// store than one or two warps, and its rounds of two elements a block fill the SMs
+// better where a round of five or eleven is followed by a short one.  us per single
+// stage (per chained one), warp / pipelined: 64 elements 4.42 / 3.60 (3.51 / 2.82),
+// 216 4.41 / 3.86 (3.61 / 3.42), 343 4.50 / 4.18 (3.70 / 4.20), 576 4.61 / 4.37, 729
+// 4.78 / 4.98, 810 5.87 / 4.96 (4.95 / 4.54), 1100 5.95 / 5.91 (5.03 / 4.71), 1452
+// 6.60 / 7.22, 1872 10.04 / 8.17 (8.74 / 7.86), 2548 10.31 / 9.88 (9.26 / 9.07), 4096
+// 13.85 / 14.32.
 inline bool warp32_few(long n, long sms, bool chained) {
-  return !chained && n > 0 &&
-         (n <= 4 * sms || (n > 5 * sms && 2 * n <= 15 * sms) || (n > 11 * sms && n <= 18 * sms));
+  return n > 0 && (2 * n <= (chained ? 3 : 8) * sms || (n > 5 * sms && 2 * n <= 15 * sms) ||
+                   (n > 11 * sms && n <= 18 * sms));
 }
 
 template <typename TQ, typename TV, typename TO, typename TC, bool EXACT,
