@@ -283,6 +283,7 @@ struct sdg_handle {
   cudaGraphExec_t graph = nullptr;       // of one step of size graph_dt
   cudaGraphExec_t graph_many = nullptr;  // of kGraphSteps of them
   double graph_dt = 0.0;
+  long long graph_steps = 0;             // steps of size graph_dt asked for so far
   // Graph of an sdg_rk3_steps_host call of host_graph_steps steps (uploads,
   // chunked stages and downloads) for the pinned host array host_graph_q
   // and host_graph_dt, and the number of kernels it launches.
@@ -627,16 +628,12 @@ void account_rk(sdg_handle* h) {
   for (auto& r : h->rk_span) account_span(h, &r);
 }
 
-// Steps of the longer step graph.  Launching one graph after another leaves a
+// The longer step graph holds kGraphSteps steps.  Launching one graph after another leaves a
 // gap that a small mesh feels, and only the kernels inside a graph overlap
 // their ends.  Measured, us per step with 1 / 2 / 4 / 8 / 16 steps a graph
 // (before the chained launches): 64 elements exact p = 7 14.4 / 12.3 / 11.8 /
 // 11.5 / 11.5, 512 elements exact p = 3 10.8 / 10.3 / 9.8 / 9.5 / 9.2; with
-// them and 8 steps a graph 10.8 and 8.8.
-constexpr int kGraphSteps = 8;
-// Calls of fewer steps take the one-step graph alone: capturing the longer one
-// costs about as much as it gives there.
-constexpr int kGraphManyFrom = 24;
+// them and 8 steps a graph 10.8 and 8.8.  Captured once step_graph_pays says so.
 
 int capture_steps(sdg_handle* h, double dt, int steps, cudaGraphExec_t* out) {
   cudaGraph_t g;
@@ -665,10 +662,12 @@ int ensure_graph(sdg_handle* h, double dt, int nsteps) {
     if (h->graph_many) cudaGraphExecDestroy(h->graph_many);
     h->graph = h->graph_many = nullptr;
     h->graph_dt = dt;
+    h->graph_steps = 0;
   }
   int rc = SDG_OK;
   if (!h->graph && (rc = capture_steps(h, dt, 1, &h->graph))) return rc;
-  if (nsteps >= kGraphManyFrom && !h->graph_many)
+  h->graph_steps += nsteps;
+  if (!h->graph_many && step_graph_pays(h->graph_steps, nsteps))
     rc = capture_steps(h, dt, kGraphSteps, &h->graph_many);
   return rc;
 }
@@ -688,6 +687,7 @@ void drop_graphs(sdg_handle* h) {
   if (h->host_graph) cudaGraphExecDestroy(h->host_graph);
   h->graph = nullptr;
   h->graph_many = nullptr;
+  h->graph_steps = 0;
   h->host_graph = nullptr;
   h->host_graph_q = nullptr;
 }
@@ -1374,7 +1374,7 @@ int sdg_rk3_steps_host(sdg_handle* h, double* q, double dt, int nsteps) {
     return sdg_get_field(h, SDG_FIELD_Q, q);
   }
   if ((rc = prime_stages(h))) return rc;
-  if (nsteps > kPlanSteps && (rc = ensure_graph(h, dt, nsteps))) return rc;
+  if (nsteps > kPlanSteps && (rc = ensure_graph(h, dt, nsteps - 2))) return rc;
   account_rk(h);
   h->have_q = true;
   const size_t NE = static_cast<size_t>(h->Np) * h->Ne;
