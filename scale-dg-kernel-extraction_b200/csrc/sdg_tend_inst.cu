@@ -38,7 +38,9 @@ int launch_kernel(void (*kern)(KArgs...), int grid, int threads, size_t smem,
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = s.pdl && pdl ? 1 : 0;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, args...));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here, not by a later launch's check
+  return static_cast<int>(e);
 }
 
 // Launches a persistent pipelined kernel: attribute and occupancy set-up on
