@@ -29,6 +29,7 @@
 // two barriers carry the verdict, so that a block leaves as one.
 #pragma once
 
+#include "sdg_in_tile.h"
 #include "sdg_tend_warp.cuh"
 
 namespace sdg {
@@ -330,10 +331,8 @@ __global__ void __launch_bounds__((LinePlan<NQ, TQ, TV, TC>::THREADS),
     for (int f = 0; f < 6; ++f) {
       const int pb = row[f];
       if (f == 1 || f == 3) {
-        const int x = pb - c.e0 * NP;
-        const bool in = pb >= 0 && x >= 0 && x < c.n * NP;
-        in_x[f == 3] = in ? x : -1;
-        if (in) continue;
+        in_x[f == 3] = node_in_tile(pb, c.e0, c.n, NP);
+        if (in_x[f == 3] >= 0) continue;
       }
       const long idx = pb >= 0 ? static_cast<long>(pb) + opp_offset<NQ>(f, a, b)
                                : static_cast<long>(-1 - pb) + n;

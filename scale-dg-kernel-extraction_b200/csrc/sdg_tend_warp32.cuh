@@ -41,6 +41,7 @@
 
 #include <cuda.h>
 
+#include "sdg_in_tile.h"
 #include "sdg_tend_warp.cuh"
 
 namespace sdg {
@@ -305,8 +306,8 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     for (int s = 0; s < 2; ++s) {
       // x: faces -x (3), +x (1); node (7 or 0, j, k) of the neighbour.
       const int p = __shfl_sync(kAll, row, s == 0 ? 3 : 1);
-      const int d = p - t.e0 * NP;
-      in_x[s] = (p >= 0 && d >= 0 && d < t.n * NP) ? d / NP : -1;
+      const int d = node_in_tile(p, t.e0, t.n, NP);
+      in_x[s] = d >= 0 ? d / NP : -1;
       if (in_x[s] < 0) {
         const long n = p >= 0 ? static_cast<long>(p) + (s == 0 ? 7 : 0) + 8 * xj + 64 * xk
                               : static_cast<long>(-1 - p) + xj + 8 * xk;
