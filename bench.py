@@ -171,6 +171,16 @@ def measured_peaks():
 STAGE_KERNEL = {"fp64_32c_p7": "tend_warp_kernel", "mixed_32c_p7": "tend_warp32_kernel"}
 
 
+def group_kernels(g):
+    """The kernel a batch's group runs and the tuned stage times (ms) by kernel.
+    At p = 7 the groups' ring variant is the warp-per-element kernel."""
+    ring = "warp" if g["p"] == 7 else "pipe"
+    names = {1: "block", 2: ring, 3: "block8", 4: "split", 6: "line"}
+    ms = {ring: g["ms_pipe"], "block": g["ms_block"], "block8": g["ms_block8"],
+          "split": g["ms_split"], "line": g["ms_line"]}
+    return names.get(g["variant"], str(g["variant"])), ms
+
+
 def profiled_traffic(workload):
     """Per-launch DRAM bytes of the fused stage kernel from the committed ncu
     summary (profiles/<kernel>_<workload>.json), or None."""
@@ -466,15 +476,13 @@ def time_batch(sdg, rep, mixed, steps, warmup, gidx, bf):
     gdof = {}
     for it in bf.comp:
         gdof[it["p"]] = gdof.get(it["p"], 0) + it["ne"] ** 3 * (it["p"] + 1) ** 3
-    names = {1: "block", 2: "pipe", 3: "block8", 4: "split"}
     groups = []
     for g in info["groups"]:
-        ms = {"pipe": g["ms_pipe"], "block": g["ms_block"], "block8": g["ms_block8"],
-              "split": g["ms_split"]}
-        chosen = ms[names.get(g["variant"], "pipe")]
+        name, ms = group_kernels(g)
+        chosen = ms.get(name, 0.0)
         gb = gdof[g["p"]] * bpd[1] / (chosen * 1e-3) / 1e9 if chosen > 0 else None
         groups.append({"p": g["p"], "dof": gdof[g["p"]], "tiles": g["tiles"],
-                       "variant": names.get(g["variant"], str(g["variant"])),
+                       "variant": name,
                        "stage2_ms": {k: round(v, 4) for k, v in ms.items() if v > 0},
                        "stage2_frac": gb / peak if gb else None})
     return {"value": value, "unit": METRIC, "ms_per_step": 1e3 * t / steps, "steps": steps,
@@ -879,7 +887,6 @@ def run_pscan(args):
     rep = Replicas("nccl", "cuda")
     import sdg_b200 as sdg
     peak, peak_kind = measured_peaks()
-    names = {1: "Block", 2: "Pipe", 3: "BlockOcc", 4: "Split"}
     orders = []
     for part in args.orders.split(","):
         lo, _, hi = part.partition("-")
@@ -903,14 +910,12 @@ def run_pscan(args):
             b.close()
             t = rep.max(i1["run_s"] - i0["run_s"])
             dof = i1["dof"]
-            g = i1["groups"][0]
+            name, ms = group_kernels(i1["groups"][0])
             bpd = sum(stage_bytes_per_dof(mixed)) / 3
             G = world * dof * 3 * args.steps / t
             rows.append({"p": p, "mixed": mixed, "mesh": N, "dof": dof,
                          "G_dof_updates_per_s": G / 1e9, "frac": G * bpd / 1e9 / peak,
-                         "variant": names.get(g["variant"], g["variant"]),
-                         "stage2_ms": {"pipe": g["ms_pipe"], "block": g["ms_block"],
-                                       "block8": g["ms_block8"], "split": g["ms_split"]}})
+                         "variant": name, "stage2_ms": ms})
     rep.close()
     if rank != 0:
         return

@@ -337,8 +337,9 @@ int sdg_batch_get(sdg_batch* b, int id, double* q);
 /* Up to n values: instances, total DOF, run seconds, DOF x steps run,
  * groups, then per group p, mixed, tiles, chosen variant and the tuned
  * stage times (ms) of the pipelined, block, 8-blocks-per-SM and
- * split-column variants (0 where not a candidate; variant 6 is the line
- * kernel, whose time is not listed).
+ * split-column variants (0 where not a candidate), and after the last group
+ * each group's tuned time of the line kernel (variant 6).  At p = 7 variant 2 of
+ * the fast FP64 and mixed forms is the warp-per-element kernel.
  * Returns the number of values available. */
 int sdg_batch_info(sdg_batch* b, double* out, int n);
 

@@ -175,7 +175,7 @@ struct Group {
   std::vector<BatchTile> h_tiles;
   cudaStream_t stream = nullptr;  // concurrent steps, autotuning, set-up
   cudaEvent_t done = nullptr;
-  double tuned_ms[5] = {0, 0, 0, 0, 0};  // by KernelVariant
+  double tuned_ms[7] = {0, 0, 0, 0, 0, 0, 0};  // by KernelVariant
 };
 
 struct Ensemble {
@@ -625,7 +625,7 @@ struct Ensemble {
         float ms = 0;
         cudaEventElapsedTime(&ms, e0, e1);
         const double t = ms / reps;
-        if (v >= 0 && v < 5) g->tuned_ms[v] = t;
+        g->tuned_ms[v] = t;
         if (t < best) {
           best = t;
           best_v = v;
@@ -828,7 +828,7 @@ int sdg_batch_get(sdg_batch* b, int id, double* q) {
 int sdg_batch_info(sdg_batch* b, double* out, int n) {
   // out: [instances, total DOF, run seconds, DOF-steps run, groups,
   //       then per group (p, mixed, tiles, variant, t_pipe, t_block, t_block8,
-  //       t_split)]
+  //       t_split), then per group t_line]
   if (!b || !out) return fail(SDG_ERR_ARG, "null argument");
   std::vector<double> v;
   long long dof = 0;
@@ -849,6 +849,7 @@ int sdg_batch_info(sdg_batch* b, double* out, int n) {
     v.push_back(g->tuned_ms[kVariantBlockOcc]);
     v.push_back(g->tuned_ms[kVariantSplit]);
   }
+  for (auto& kv : b->ens.groups) v.push_back(kv.second->tuned_ms[kVariantLine]);
   for (int i = 0; i < n && i < static_cast<int>(v.size()); ++i) out[i] = v[i];
   return static_cast<int>(v.size());
 }

@@ -580,12 +580,13 @@ class Batch:
         buf = np.zeros(512)
         n = lib().sdg_batch_info(self._b, _p(buf), 512)
         v = buf[:n]
-        groups = []
-        for g in range(int(v[4])):
+        groups, ng = [], int(v[4])
+        for g in range(ng):
             r = v[5 + 8 * g: 13 + 8 * g]
             groups.append({"p": int(r[0]), "mixed": bool(r[1]), "tiles": int(r[2]),
                            "variant": int(r[3]), "ms_pipe": r[4], "ms_block": r[5],
-                           "ms_block8": r[6], "ms_split": r[7]})
+                           "ms_block8": r[6], "ms_split": r[7],
+                           "ms_line": v[5 + 8 * ng + g]})
         return {"instances": int(v[0]), "dof": int(v[1]), "run_s": v[2],
                 "dof_steps": int(v[3]), "groups": groups}
 
