@@ -192,10 +192,11 @@ constexpr int kSplitH = 2;
 // p = 11 0.251 / 0.325, p = 12 0.246 / 0.316, p = 13 0.252 / 0.295; mixed
 // p = 8 0.129 / 0.146, p = 9 0.144 / 0.158, p = 11 0.132 / 0.146.  Slower at
 // FP64 p = 10 and 14 (0.232 / 0.230, 0.332 / 0.313) and the other mixed
-// orders.
+// orders.  At FP64 p = 9, 11 and 12 the line kernel leaves it the single stages of
+// few elements (line_few); p = 13 is the line kernel's at every size.
 template <int NQ, typename TC, bool EXACT>
 constexpr bool kSplitAuto =
-    !EXACT && (sizeof(TC) == 8 ? (NQ == 9 || NQ == 10 || (NQ >= 12 && NQ <= 14))
+    !EXACT && (sizeof(TC) == 8 ? (NQ == 9 || NQ == 10 || NQ == 12 || NQ == 13)
                                : (NQ == 9 || NQ == 10 || NQ == 12));
 
 // Blocks per SM the kernel is built for: what the shared memory allows,
