@@ -51,12 +51,17 @@ namespace {
 // compiler's own choice (0), us for 7.4 M values, gradient / five fields: p = 11
 // 61.5 / 65.8 with three blocks (66.8 / 72.0), p = 13 83 / 94 with two and the z
 // contraction first (109 / 112: 254 registers, one block of seven warps).
-// Elsewhere one to eight blocks measured no better.
+// Elsewhere one to eight blocks measured no better.  Calls of few units keep the
+// compiler's choice, which is faster where the blocks do not fill the SMs: us of a
+// gradient at 148 SMs, p = 11 148 units 4.49 / 4.75, 296 5.89 / 6.19, 300 8.03 / 7.11;
+// p = 13 148 6.26 / 6.74, 200 10.63 / 9.51.
 template <int NQ, bool EXACT>
 constexpr int kDerivBlocks = EXACT ? 0 : NQ == 12 ? 3 : NQ == 14 ? 2 : 0;
+template <int NQ>
+constexpr int kDerivFewPerSm = NQ == 12 ? 2 : 1;
 
-template <int NQ, bool EXACT, int ORDER, bool ONE>
-__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, kDerivBlocks<NQ, EXACT>)
+template <int NQ, bool EXACT, int ORDER, bool ONE, int BLOCKS>
+__global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, BLOCKS)
     derivative_kernel(const double* __restrict__ ix, const double* __restrict__ iy,
                       const double* __restrict__ iz, double* __restrict__ ox,
                       double* __restrict__ oy, double* __restrict__ oz, long long units,
@@ -88,7 +93,7 @@ __global__ void __launch_bounds__((Geo<NQ>::THREADS + 31) / 32 * 32, kDerivBlock
   // 109-146 / 93-133; five fields p = 7 125 / 144, p = 8 115 / 125, p = 9
   // 112 / 119; both p = 14 76-81 / 135-155.
   constexpr bool EARLYZ = (NQ >= 11 && NQ <= 13) || (ONE && (NQ == 9 || NQ == 10)) ||
-                          (NQ == 14 && !EXACT);
+                          (NQ == 14 && BLOCKS > 0);
   auto zderiv = [&](const double (&col)[NQ]) {
     // Z-dir (erb:430-463): vec_in_z(i,j,l) * Mat_tr(l,k), stored straight
     // from registers (coalesced over the warp).
@@ -257,6 +262,20 @@ int launch_units(const DerivCall& c, int buffers) {
   return SDG_OK;
 }
 
+// Multiprocessors of the current device.
+int sm_count() {
+  static DeviceSetup setup;  // per device
+  const int dev = setup_device();
+  if (dev < 0) return 148;
+  int n = setup.slot[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 148;
+    setup.slot[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 template <int NQ, bool EXACT, int ORDER, bool ONE>
 int launch_derivative(const DerivCall& c) {
   if constexpr (kDerivHalf<NQ, EXACT, ONE>) {
@@ -269,7 +288,12 @@ int launch_derivative(const DerivCall& c) {
       for (const double* o : out) apart = apart && (o + n <= i || i + n <= o);
     if (apart) return launch_units<derivative_half_kernel<NQ, ORDER, ONE>, NQ>(c, 1);
   }
-  return launch_units<derivative_kernel<NQ, EXACT, ORDER, ONE>, NQ>(c, 2);
+  if constexpr (kDerivBlocks<NQ, EXACT> > 0) {
+    if (c.units > static_cast<long long>(kDerivFewPerSm<NQ>) * sm_count())
+      return launch_units<derivative_kernel<NQ, EXACT, ORDER, ONE, kDerivBlocks<NQ, EXACT>>, NQ>(
+          c, 2);
+  }
+  return launch_units<derivative_kernel<NQ, EXACT, ORDER, ONE, 0>, NQ>(c, 2);
 }
 
 template <int NQ>
