@@ -268,9 +268,14 @@ int run(const LaunchSpec& s) {
                                       : line_few<NQ, TC, EXACT, STAGE>(s.nelem, sms, s.pdl,
                                                                        s.nelem < s.Ne));
     if (can && (s.variant == kVariantLine || (s.variant == kVariantAuto && !batch))) {
-      // Shorter tiles where the longest would leave a block without one.
+      // Shorter tiles where the longest would leave a block without one; not at Nq = 2,
+      // whose elements are small: blocks of a few elements fill the SMs without using
+      // them, and stages of other handles wait.  us per step of one handle / of four
+      // side by side, tiles spread / full: 1,000 elements 7.3 / 3.0 and 8.1 / 2.4, 4,046
+      // 8.6 / 7.5 and 9.3 / 2.9, 8,000 9.0 / 7.6 and 10.3 / 4.0 (the kernel before 14.7 / 5.4).
       const int slots = LineTile<NQ, TC>::BLOCKS * sms;
-      a.tile_elems = std::max(1, std::min(LP::E, (s.nelem + slots - 1) / slots));
+      a.tile_elems =
+          NQ == 2 ? LP::E : std::max(1, std::min(LP::E, (s.nelem + slots - 1) / slots));
       const int ntiles = batch ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
       if (batch)
         return launch_pipe<tend_line_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, true>,
