@@ -78,7 +78,8 @@ int launch_pipe(size_t smem, int ntiles, const LaunchSpec& s, const Args& a, con
 
 // Launches the warp-per-element kernel with H warps an element and tiles of E
 // elements, or fewer where that leaves an SM without one: one block per SM, or
-// one per tile where there are fewer.
+// one per tile where there are fewer.  Chained stages of one warp an element keep
+// full tiles, which leave SMs to other handles (warp_form).
 template <bool STAGE, bool BATCH, bool VEC, int H, int E, typename Args, typename Dm>
 int launch_warp(const LaunchSpec& s, Args& a, const Dm& d) {
   constexpr auto kern = tend_warp_kernel<STAGE, BATCH, VEC, H, E>;
@@ -94,7 +95,8 @@ int launch_warp(const LaunchSpec& s, Args& a, const Dm& d) {
     setup.slot[dev].store(1, std::memory_order_relaxed);
   }
   const int sms = s.num_sms > 0 ? s.num_sms : 148;
-  a.tile_elems = std::max(1, std::min(E, (s.nelem + sms - 1) / sms));
+  a.tile_elems =
+      s.pdl && H == 1 ? E : std::max(1, std::min(E, (s.nelem + sms - 1) / sms));
   const int ntiles = BATCH ? s.batch_ntiles : (s.nelem + a.tile_elems - 1) / a.tile_elems;
   if (ntiles <= 0) return 0;
   return launch_kernel(kern, std::min(ntiles, sms), P::THREADS, P::BYTES, s, true, a, d);
@@ -132,8 +134,16 @@ int launch_warp32(const LaunchSpec& s, Args& a, const Dm& d, const FieldMaps& m)
 // (2,3) 252 5.11 / 3.86, 392 5.10 / 3.95; (2,4) 392 5.59 / 4.47, 576 5.62 / 4.62, 1100
 // 8.64 / 7.29; (1,7) 576 6.38 / 5.23, 729 6.47 / 5.36, 1100 10.14 / 8.25.  (Nine
 // warps leave a thread 168 registers instead of 255.)
+//
+// Chained stages, of which a program may have several handles' in flight, split only
+// where the blocks of a few handles still fit side by side: a split element takes
+// two to three times the SM time.  us per step of one handle / of four, this rule /
+// split forms: 64 elements 8.2 / 3.9, 125 14.4 / 4.0 and 9.4 / 7.3, 343 14.1 / 5.2 and
+// 12.7 / 9.0 (the pipelined kernel of this form before: 17.0 / 5.1, 19.1 / 6.9).
 enum class WarpForm { k41, k42, k23, k24, k17 };
-inline WarpForm warp_form(int per_sm) {
+inline WarpForm warp_form(long n, long sms, bool chained) {
+  if (chained) return 2 * n <= sms ? WarpForm::k41 : WarpForm::k17;
+  const long per_sm = (n + sms - 1) / sms;
   return per_sm <= 1   ? WarpForm::k41
          : per_sm == 2 ? WarpForm::k42
          : per_sm == 3 ? WarpForm::k23
@@ -142,18 +152,22 @@ inline WarpForm warp_form(int per_sm) {
 }
 
 // Mixed form at Nq = 8: whether a launch of n elements stays with the pipelined
-// kernel: its 64 threads an element have a shorter way from the first copy to the
-// store than one or two warps, and its rounds of two elements a block fill the SMs
-// better where a round of five or eleven is followed by a short one.  us per single
-// stage (per chained one), warp / pipelined: 64 elements 4.42 / 3.60 (3.51 / 2.82),
-// 216 4.41 / 3.86 (3.61 / 3.42), 343 4.50 / 4.18 (3.70 / 4.20), 576 4.61 / 4.37, 729
-// 4.78 / 4.98, 810 5.87 / 4.96 (4.95 / 4.54), 1100 5.95 / 5.91 (5.03 / 4.71), 1452
-// 6.60 / 7.22, 1872 10.04 / 8.17 (8.74 / 7.86), 2548 10.31 / 9.88 (9.26 / 9.07), 4096
-// 13.85 / 14.32.
-inline bool warp32_few(long n, long sms, bool chained) {
-  return n > 0 && (2 * n <= (chained ? 3 : 8) * sms || (n > 5 * sms && 2 * n <= 15 * sms) ||
-                   (n > 11 * sms && n <= 18 * sms));
-}
+// kernel.  Its 64 threads an element have a shorter way from the first copy to the
+// store than one warp, its rounds of two elements a block fill the SMs better than
+// rounds of eleven where there are few, and its blocks leave room for other handles'
+// where a block of eleven warps takes an SM.  us per single stage, warp / pipelined:
+// 64 elements 4.42 / 3.60, 810 5.87 / 4.96, 1872 10.04 / 8.17, 4096 13.85 / 14.32; per
+// step of one handle / of four: 343 12.4 / 8.4 and 12.7 / 4.0, 1331 16.8 / 15.4 and 18.2 /
+// 13.2, 4096 40.8 / 42.7 and 44.4 / 39.5, 8000 69.0 / 70.4 and 78.3 / 66.2, 13824 119.6 /
+// 109.9 and 129.1 / 115.6.
+inline bool warp32_few(long n, long sms) { return n > 0 && n <= 64 * sms; }
+
+// Chained launches of the pipelined kernel: up to this many nodes.  Starting early
+// saves about a microsecond a launch, which small meshes feel; but the blocks that
+// wait hold their SMs, which other handles' launches feel (three handles, us per
+// call: FP64 27,000 elements p = 2, ten steps 356 chained, 353 not; mixed p = 2 414,504
+// elements, two steps 835 and 823).
+constexpr long kChainNodes = 500000;
 
 template <typename TQ, typename TV, typename TO, typename TC, bool EXACT,
           int ORDER, bool STAGE>
@@ -216,7 +230,7 @@ int run(const LaunchSpec& s) {
       if (batch) return launch_warp<STAGE, true, true, 1, kWarpElems>(s, a, d);
       if (!vec) return launch_warp<STAGE, false, false, 1, kWarpElems>(s, a, d);
       const int sms = s.num_sms > 0 ? s.num_sms : 148;
-      const WarpForm form = warp_form((s.nelem + sms - 1) / sms);
+      const WarpForm form = warp_form(s.nelem, sms, s.pdl);
       const bool prime = s.nelem <= 0;  // a call without elements primes every form
       int rc = 0;
       auto take = [&](WarpForm f, auto launch) {
@@ -234,7 +248,7 @@ int run(const LaunchSpec& s) {
   if constexpr (STAGE && kWarp32Kernel<NQ, TC, EXACT>) {
     if (s.lift_z != nullptr &&
         (batch || (s.field_maps != nullptr && s.variant == kVariantAuto &&
-                   !warp32_few(s.nelem, s.num_sms > 0 ? s.num_sms : 148, s.pdl))) &&
+                   !warp32_few(s.nelem, s.num_sms > 0 ? s.num_sms : 148))) &&
         Warp32Plan<TQ, 1>::BYTES <= device_smem_optin()) {
       FieldMaps m;
       std::memset(&m, 0, sizeof(m));
@@ -347,7 +361,8 @@ int run(const LaunchSpec& s) {
     // 2-4 % (mixed p = 5, 256,000 nodes 4.60 -> 4.80 us).  (A call without
     // elements primes both.)
     if constexpr (PDL) {
-      if (s.pdl || s.nelem <= 0) {
+      const bool chain = s.pdl && static_cast<long>(s.nelem) * G::NP <= kChainNodes;
+      if (chain || s.nelem <= 0) {
         const int rc = launch_pipe<
             tend_pipe_kernel<NQ, TQ, TV, TO, TC, EXACT, ORDER, STAGE, false, false, true>>(
             P::BYTES, ntiles, s, a, d, 0, true);
