@@ -104,10 +104,10 @@ int launch_warp(const LaunchSpec& s, Args& a, const Dm& d) {
 
 // The mixed form's warp-per-element kernel: tiles of the most elements a slot
 // holds, or fewer where that leaves an SM without one.
-template <auto KERN, typename TQ, int H, typename Args, typename Dm>
+template <auto KERN, typename TQ, typename Args, typename Dm>
 int launch_warp32(const LaunchSpec& s, Args& a, const Dm& d, const FieldMaps& m) {
   constexpr auto kern = KERN;
-  using P = Warp32Plan<TQ, H>;
+  using P = Warp32Plan<TQ>;
   static DeviceSetup setup;  // per kernel and device
   const int dev = setup_device();
   if (dev < 0) return static_cast<int>(cudaErrorInvalidDevice);
@@ -249,23 +249,14 @@ int run(const LaunchSpec& s) {
     if (s.lift_z != nullptr &&
         (batch || (s.field_maps != nullptr && s.variant == kVariantAuto &&
                    !warp32_few(s.nelem, s.num_sms > 0 ? s.num_sms : 148))) &&
-        Warp32Plan<TQ, 1>::BYTES <= device_smem_optin()) {
+        Warp32Plan<TQ>::BYTES <= device_smem_optin()) {
       FieldMaps m;
       std::memset(&m, 0, sizeof(m));
-      if (batch) return launch_warp32<tend_warp32_kernel<TQ, TO, true, 1>, TQ, 1>(s, a, d, m);
+      if (batch) return launch_warp32<tend_warp32_kernel<TQ, TO, true>, TQ>(s, a, d, m);
       std::memcpy(&m, s.field_maps, sizeof(m));
-      // Two warps an element while one round of tiles of five holds the mesh:
-      // us per RK step with one / two warps, 64 elements 18.7 / 14.6, 740 18.6
-      // / 14.6, 888 18.6 / 20.7, 1628 20.7 / 28.9.  (A call without elements
-      // primes both forms and the kernel of warp32_few.)
-      const int sms = s.num_sms > 0 ? s.num_sms : 148;
-      const bool split = s.nelem <= sms * Warp32Plan<TQ, 2>::ELEMS;
-      int rc = 0;
-      if (split || s.nelem <= 0)
-        rc = launch_warp32<tend_warp32_kernel<TQ, TO, false, 2>, TQ, 2>(s, a, d, m);
-      if (rc == 0 && (!split || s.nelem <= 0))
-        rc = launch_warp32<tend_warp32_kernel<TQ, TO, false, 1>, TQ, 1>(s, a, d, m);
+      const int rc = launch_warp32<tend_warp32_kernel<TQ, TO, false>, TQ>(s, a, d, m);
       if (rc != 0 || s.nelem > 0) return rc;
+      // (A call without elements primes this kernel and the one of warp32_few.)
     }
   }
   // The line kernel.
@@ -446,7 +437,7 @@ int pipe_fits() {
     if (WarpPlan<1, kWarpElems>::BYTES <= optin) r |= 4;
   }
   if constexpr (STAGE && kWarp32Kernel<NQ, TC, false>) {
-    if (Warp32Plan<TQ, 1>::BYTES <= optin) r |= 4;
+    if (Warp32Plan<TQ>::BYTES <= optin) r |= 4;
   }
   if constexpr (kLineAuto<NQ, TC, false> || kLineAuto<NQ, TC, true>) {
     if (LinePlan<NQ, TQ, TV, TC>::BYTES <= optin)

@@ -33,10 +33,8 @@
 // 168 registers measured better than fourteen of 128 (8 KB an element: the
 // slots would hold them), which spill.
 //
-// H = 2 warps per element, a line a lane instead of two: the latency form for
-// meshes too small to give every warp of the GPU an element.  The packed
-// instructions round each half as the scalar ones, so the results do not
-// depend on H.
+// It takes the batch and meshes of more than 64 elements an SM; smaller ones stay with
+// tend_pipe_kernel (warp32_few).
 #pragma once
 
 #include <cuda.h>
@@ -56,14 +54,14 @@ struct alignas(64) FieldMaps {
 };
 static_assert(sizeof(FieldMaps) == kFieldMapsBytes, "FieldMaps");
 
-template <typename TQ, int H>
+template <typename TQ>
 struct Warp32Plan {
   static constexpr int NP = 512;
   static constexpr size_t QB = NP * sizeof(TQ);
   static constexpr size_t VB = NP * sizeof(float);
   static constexpr size_t ELEM = QB + 3 * VB;     // 8 KB, 10 KB with FP64 q
-  static constexpr int ELEMS = kWarpElems32 / H;  // per tile at most
-  static constexpr int WARPS = ELEMS * H;          // consumer warps
+  static constexpr int ELEMS = kWarpElems32;  // per tile at most
+  static constexpr int WARPS = ELEMS;         // consumer warps
   static constexpr int NSTAGE = 2;
   static constexpr int THREADS = 32 * (WARPS + 1);
   static constexpr size_t SLOT = ELEMS * ELEM;
@@ -71,8 +69,8 @@ struct Warp32Plan {
   static constexpr size_t OFF_C = NSTAGE * SLOT + 16 * NSTAGE;
   static constexpr size_t BYTES = OFF_C + 4 * 128 + 1024;  // contexts as in WarpPlan
 };
-static_assert(Warp32Plan<float, 1>::BYTES <= kPipeMaxSmem &&
-                  Warp32Plan<double, 1>::BYTES <= kPipeMaxSmem,
+static_assert(Warp32Plan<float>::BYTES <= kPipeMaxSmem &&
+                  Warp32Plan<double>::BYTES <= kPipeMaxSmem,
               "warp kernel: shared memory");
 
 // Tiled copy of the map's box at row `row` (no multicast); dst 128-byte
@@ -104,8 +102,7 @@ __device__ __forceinline__ int swz(int i, int j, int k) {
   }
 }
 
-// The value of a lane's line or, packed, of its two lines.
-template <int H>
+// A value of a lane's two lines, packed.
 struct Lines {
   using V = float2;
   static __device__ __forceinline__ V make(float a, float b) { return make_float2(a, b); }
@@ -129,25 +126,6 @@ struct Lines {
   }
   static __device__ __forceinline__ void st(float* p, V a) { *reinterpret_cast<float2*>(p) = a; }
 };
-template <>
-struct Lines<2> {
-  using V = float;
-  static __device__ __forceinline__ V make(float a, float) { return a; }
-  static __device__ __forceinline__ float lo(V a) { return a; }
-  static __device__ __forceinline__ float hi(V a) { return a; }
-  static __device__ __forceinline__ V dup(float a) { return a; }
-  static __device__ __forceinline__ V mul(V a, V b) { return __fmul_rn(a, b); }
-  static __device__ __forceinline__ V add(V a, V b) { return __fadd_rn(a, b); }
-  static __device__ __forceinline__ V fma(V a, V b, V c) { return fmaf(a, b, c); }
-  static __device__ __forceinline__ V neg(V a) { return -a; }
-  static __device__ __forceinline__ V abs(V a) { return fabsf(a); }
-  static __device__ __forceinline__ V sub_products(V a, V b, V c, V d) {
-    return __fsub_rn(__fmul_rn(a, b), __fmul_rn(c, d));
-  }
-  static __device__ __forceinline__ V ld(const float* p) { return *p; }
-  static __device__ __forceinline__ void st(float* p, V a) { *p = a; }
-};
-
 __device__ __forceinline__ float ld_early(const float* p) {
   float v;
   asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
@@ -159,16 +137,15 @@ __device__ __forceinline__ float ld_early_state(const float* p) {
   return v;
 }
 
-template <typename TQ, typename TO, bool BATCH, int H>
-__global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
+template <typename TQ, typename TO, bool BATCH>
+__global__ void __launch_bounds__(Warp32Plan<TQ>::THREADS, 1)
     tend_warp32_kernel(const __grid_constant__ TendArgs<TQ, float, TO, float> A,
                        const __grid_constant__ DMat<8, float> D,
                        const __grid_constant__ FieldMaps M) {
-  using P = Warp32Plan<TQ, H>;
+  using P = Warp32Plan<TQ>;
   using Ctx = TileCtx<TQ, float, TO, float>;
-  using L = Lines<H>;
+  using L = Lines;
   using V = typename L::V;
-  constexpr bool PAIR = H == 1;  // two lines a lane
   constexpr int NP = P::NP;
   constexpr int NS = P::NSTAGE;
   constexpr unsigned kAll = 0xffffffffu;
@@ -179,8 +156,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
   uint64_t* empty = full + NS;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int es = warp / H;              // element of the tile
-  const int hw = H == 1 ? 0 : warp % H; // half of the lines
+  const int es = warp;  // element of the tile
   const int tw = A.tile_elems;  // elements per tile (single instance)
   const int ntiles = BATCH ? A.ntiles : (A.nelem + tw - 1) / tw;
   auto context = [&](int tile) {
@@ -191,12 +167,6 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     }
     return t;
   };
-  // Between the phases: the warps of an element.
-  auto sync_elem = [&]() {
-    if constexpr (H == 1) __syncwarp();
-    else bar_sync_warps(1 + es, 32 * H);
-  };
-
   if (threadIdx.x == 0) {
     for (int k = 0; k < NS; ++k) {
       mbar_init(&full[k], 1);
@@ -270,15 +240,15 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     return;
   }
 
-  // This lane's lines: x (xj, xk [, xk + 4]); y (yi [, yi + 1], yk); z (yi [,
-  // yi + 1], zj).
-  const int xj = lane & 7, xk = (lane >> 3) + 4 * hw;
-  const int yi = PAIR ? 2 * (lane & 3) : lane & 7;
-  const int yk = PAIR ? lane >> 2 : (lane >> 3) + 4 * hw;
+  // This lane's lines: x (xj, xk), (xj, xk + 4); y (yi, yk), (yi + 1, yk); z (yi, zj),
+  // (yi + 1, zj).
+  const int xj = lane & 7, xk = lane >> 3;
+  const int yi = 2 * (lane & 3);
+  const int yk = lane >> 2;
   const int zj = yk;
   // Lift factors of the faces +x and -x at this lane's i.
-  const V lx2 = L::make(D.lx[8 + yi], PAIR ? D.lx[9 + yi] : 0.0f);
-  const V lx4 = L::make(D.lx[yi], PAIR ? D.lx[1 + yi] : 0.0f);
+  const V lx2 = L::make(D.lx[8 + yi], D.lx[9 + yi]);
+  const V lx4 = L::make(D.lx[yi], D.lx[1 + yi]);
 
   // Face-neighbour row and metric factors, one word per lane, a tile ahead.
   auto load_row = [&](const Ctx& t, int* row, float* met) {
@@ -291,15 +261,14 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
   // of the tile, else -1).
   V xq[2], xu[2], yq[2], yv[2], zq[2], zw[2];
   int in_x[2] = {-1, -1};
-  // Two values at p and p + d (one where the lane has one line): of a velocity,
-  // of the state.
+  // Two values at p and p + d: of a velocity, of the state.
   auto early = [&](const float* p, int d) {
     const float a = ld_early(p);
-    return L::make(a, PAIR ? ld_early(p + d) : 0.0f);
+    return L::make(a, ld_early(p + d));
   };
   auto early_state = [&](const TQ* p, int d) {
     const float a = static_cast<float>(ld_early_state(p));
-    return L::make(a, PAIR ? static_cast<float>(ld_early_state(p + d)) : 0.0f);
+    return L::make(a, static_cast<float>(ld_early_state(p + d)));
   };
   auto gather = [&](const Ctx& t, int row) {
 #pragma unroll
@@ -330,7 +299,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       // z: faces -z (4), +z (5); nodes (i; j; 7 or 0).
       const int p = __shfl_sync(kAll, row, 4 + s);
       const long n = (p >= 0 ? static_cast<long>(p) + (s == 0 ? 448 : 0)
-                             : static_cast<long>(-1 - p)) + (PAIR ? 2 * lane : 8 * zj + yi);
+                             : static_cast<long>(-1 - p)) + 2 * lane;
       zq[s] = early_state(t.q + n, 1);
       zw[s] = early(t.w + n, 1);
     }
@@ -346,11 +315,9 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
   auto ld_q = [](const TQ* p) {
     if constexpr (sizeof(TQ) == 4) {
       return L::ld(reinterpret_cast<const float*>(p));
-    } else if constexpr (PAIR) {
+    } else {
       const double2 v = *reinterpret_cast<const double2*>(p);
       return L::make(static_cast<float>(v.x), static_cast<float>(v.y));
-    } else {
-      return L::make(static_cast<float>(*p), 0.0f);
     }
   };
 
@@ -377,8 +344,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     if constexpr (BATCH) {  // the contexts come with the copies
       const uint32_t parity = (it / NS) & 1;
       const bool ok = mbar_wait_bounded(&full[slot], parity, A.wait_spins);
-      // The warps that share an element leave together, or none does.
-      if (!(H == 1 ? __all_sync(kAll, ok) != 0 : bar_and_warps(1 + es, 32 * H, ok))) {
+      if (__all_sync(kAll, ok) == 0) {
         // Wait for the copies still in flight (bounded) and leave.
         if (lane == 0) {
           atomicExch(A.status, kStatusWaitTimeout);
@@ -391,7 +357,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     const Ctx C = of_tile(it, tile);
     const Ctx N = more ? of_tile(it + 1, tile + gridDim.x) : C;
     const bool active = es < C.n;  // idle warps of a short tile keep pace
-    const long base = static_cast<long>(C.e0 + (active ? es : 0)) * NP + (PAIR ? 2 * lane : 8 * zj + yi);
+    const long base = static_cast<long>(C.e0 + (active ? es : 0)) * NP + 2 * lane;
     unsigned char* st = smem + slot * P::SLOT;
     unsigned char* sb = st + es * P::ELEM;
     const TQ* sq = reinterpret_cast<const TQ*>(sb);
@@ -411,8 +377,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     if constexpr (!BATCH) {
       const uint32_t parity = (it / NS) & 1;
       const bool ok = mbar_wait_bounded(&full[slot], parity, A.wait_spins);
-      // The warps that share an element leave together, or none does.
-      if (!(H == 1 ? __all_sync(kAll, ok) != 0 : bar_and_warps(1 + es, 32 * H, ok))) {
+      if (__all_sync(kAll, ok) == 0) {
         // Wait for the copies still in flight (bounded) and leave.
         if (lane == 0) {
           atomicExch(A.status, kStatusWaitTimeout);
@@ -432,8 +397,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       V q2;
       const TQ* pq = sq + swz<TQ>(yi, zj, k);
       if constexpr (sizeof(TQ) == 8) {
-        if constexpr (PAIR) qd[k] = *reinterpret_cast<const double2*>(pq);
-        else qd[k].x = *pq;
+        qd[k] = *reinterpret_cast<const double2*>(pq);
         q2 = L::make(static_cast<float>(qd[k].x), static_cast<float>(qd[k].y));
       } else {
         q2 = qf[k] = ld_q(pq);
@@ -443,7 +407,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       if (k == 7) { qh = q2; wh = w2; }
       fz[k] = L::mul(q2, w2);
     }
-    sync_elem();
+    __syncwarp();
 
     // ---- x-lines -------------------------------------------------------------
     {
@@ -456,20 +420,20 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
           for (int m = 0; m < 2; ++m) {
             const double2 x = *reinterpret_cast<const double2*>(sq + swz<TQ>(4 * h + 2 * m, xj, xk));
             const double2 y =
-                PAIR ? *reinterpret_cast<const double2*>(sq + swz<TQ>(4 * h + 2 * m, xj, xk + 4)) : x;
+                *reinterpret_cast<const double2*>(sq + swz<TQ>(4 * h + 2 * m, xj, xk + 4));
             q[2 * m] = L::make(static_cast<float>(x.x), static_cast<float>(y.x));
             q[2 * m + 1] = L::make(static_cast<float>(x.y), static_cast<float>(y.y));
           }
         } else {
           const float4 x = *reinterpret_cast<const float4*>(sq + swz<TQ>(4 * h, xj, xk));
           const float4 y =
-              PAIR ? *reinterpret_cast<const float4*>(sq + swz<TQ>(4 * h, xj, xk + 4)) : x;
+              *reinterpret_cast<const float4*>(sq + swz<TQ>(4 * h, xj, xk + 4));
           q[0] = L::make(x.x, y.x); q[1] = L::make(x.y, y.y);
           q[2] = L::make(x.z, y.z); q[3] = L::make(x.w, y.w);
         }
         const float4 ua = *reinterpret_cast<const float4*>(su + swz<float>(4 * h, xj, xk));
         const float4 ub =
-            PAIR ? *reinterpret_cast<const float4*>(su + swz<float>(4 * h, xj, xk + 4)) : ua;
+            *reinterpret_cast<const float4*>(su + swz<float>(4 * h, xj, xk + 4));
         u[0] = L::make(ua.x, ub.x); u[1] = L::make(ua.y, ub.y);
         u[2] = L::make(ua.z, ub.z); u[3] = L::make(ua.w, ub.w);
 #pragma unroll
@@ -492,24 +456,22 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
           const float* nu = reinterpret_cast<const float*>(nb + P::QB);
           const int i = s == 0 ? 7 : 0;
           xq[s] = L::make(static_cast<float>(nq[swz<TQ>(i, xj, xk)]),
-                          PAIR ? static_cast<float>(nq[swz<TQ>(i, xj, xk + 4)]) : 0.0f);
-          xu[s] = L::make(nu[swz<float>(i, xj, xk)], PAIR ? nu[swz<float>(i, xj, xk + 4)] : 0.0f);
+                          static_cast<float>(nq[swz<TQ>(i, xj, xk + 4)]));
+          xu[s] = L::make(nu[swz<float>(i, xj, xk)], nu[swz<float>(i, xj, xk + 4)]);
         }
       // (f2, f4) of this line over nodes 2, 3 of its u: a neighbour reads only
       // the ends.
       const V f4 = flux(q0e, u0e, xq[0], xu[0], true, hs[3]);
       const V f2 = flux(q7e, u7e, xq[1], xu[1], false, hs[1]);
       *reinterpret_cast<float2*>(su + swz<float>(2, xj, xk)) = make_float2(L::lo(f2), L::lo(f4));
-      if constexpr (PAIR)
-        *reinterpret_cast<float2*>(su + swz<float>(2, xj, xk + 4)) =
-            make_float2(L::hi(f2), L::hi(f4));
+      *reinterpret_cast<float2*>(su + swz<float>(2, xj, xk + 4)) =
+          make_float2(L::hi(f2), L::hi(f4));
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         *reinterpret_cast<float4*>(sw + swz<float>(4 * h, xj, xk)) = make_float4(
             L::lo(r[4 * h]), L::lo(r[4 * h + 1]), L::lo(r[4 * h + 2]), L::lo(r[4 * h + 3]));
-        if constexpr (PAIR)
-          *reinterpret_cast<float4*>(sw + swz<float>(4 * h, xj, xk + 4)) = make_float4(
-              L::hi(r[4 * h]), L::hi(r[4 * h + 1]), L::hi(r[4 * h + 2]), L::hi(r[4 * h + 3]));
+        *reinterpret_cast<float4*>(sw + swz<float>(4 * h, xj, xk + 4)) = make_float4(
+            L::hi(r[4 * h]), L::hi(r[4 * h + 1]), L::hi(r[4 * h + 2]), L::hi(r[4 * h + 3]));
       }
     }
     // q0 (in L2 since the tile's copies were issued).
@@ -517,12 +479,9 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
     double2 q0[kQ0 ? 8 : 1];
     if constexpr (kQ0) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        if constexpr (PAIR) q0[k] = ld_early_stream2(C.q0 + base + 64 * k);
-        else q0[k].x = __ldcs(C.q0 + base + 64 * k);
-      }
+      for (int k = 0; k < 8; ++k) q0[k] = ld_early_stream2(C.q0 + base + 64 * k);
     }
-    sync_elem();
+    __syncwarp();
 
     // ---- y-lines ---------------------------------------------------------------
     {
@@ -553,7 +512,7 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
         L::st(sv + swz<float>(yi, j, yk), lf);
       }
     }
-    sync_elem();
+    __syncwarp();
 
     // ---- z-lines ---------------------------------------------------------------
     const V f5 = flux(ql, wl, zq[0], zw[0], true, hs[4]);
@@ -596,14 +555,12 @@ __global__ void __launch_bounds__(Warp32Plan<TQ, H>::THREADS, 1)
       }
       const float a[2] = {-L::lo(acc[k]), -L::hi(acc[k])};
 #pragma unroll
-      for (int m = 0; m < (PAIR ? 2 : 1); ++m) {
+      for (int m = 0; m < 2; ++m) {
         r[m] = AD::mul(A.rk_b, AD::mad(C.dt, static_cast<double>(a[m]), q2[m]));
         if constexpr (kQ0) r[m] = AD::mad(A.rk_a, m == 0 ? q0[k].x : q0[k].y, r[m]);
       }
       TO* o = C.out + base + 64 * k;
-      if constexpr (!PAIR)
-        *o = static_cast<TO>(r[0]);
-      else if constexpr (sizeof(TO) == 8)
+      if constexpr (sizeof(TO) == 8)
         *reinterpret_cast<double2*>(o) = make_double2(r[0], r[1]);
       else
         *reinterpret_cast<float2*>(o) =
