@@ -44,9 +44,10 @@
 // 3 and 375 us a chained step, against 153 / 160 / 160 and 469 for the block kernel
 // it replaced (two warps per element, line buffers and fluxes in shared memory); the
 // step is 6.1 TB/s of the 40 / 48 / 48 algorithmic bytes per node, where a copy
-// reaches 6.56.  Tried on the way: seven independent warps with a ring each and all
-// face values from L2, 153 / 183 / 183 (the -x/+x faces are 8-byte words 64 bytes
-// apart, each a 32-byte sector); without any neighbour's values 111 / 130.
+// reaches 6.56.  Shared-memory pipe 75 -> 38 % busy; seven warps per SM, about 1,100
+// instructions per element.  Tried on the way: seven independent warps with a ring
+// each and all face values from L2, 153 / 183 / 183 (the -x/+x faces are 8-byte words
+// 64 bytes apart, each a 32-byte sector); without any neighbour's values 111 / 130.
 //
 // H warps per element (1, 2 or 4): the latency form for meshes too small to
 // give every warp of the GPU an element.  Warp h of an element takes planes
